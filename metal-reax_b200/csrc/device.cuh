@@ -246,6 +246,26 @@ __device__ inline double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+// Sums of NV values (a power of two, 2 to 32) over the warp with NV - 1 + log2(32 / NV) exchanges instead of 5 NV: at each
+// of the first log2(NV) steps a lane keeps half of its values and hands the other half over. Lane l returns the total
+// of value l / (32 / NV). The order of the additions is fixed.
+template <int NV>
+__device__ inline double warp_sums(double* v) {
+  const int lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int m = NV / 2; m > 0; m >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int k = 0; k < m; ++k) {
+      const double give = up ? v[k] : v[k + m];
+      const double keep = up ? v[k + m] : v[k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
 __device__ inline float warp_sumf(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
