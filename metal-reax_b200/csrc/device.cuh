@@ -96,7 +96,14 @@ struct Dev {
   double* q;             // charges
   // cells
   int* cell_key;         // global cell of every atom (sort key)
+  // Cell order: position p holds atom cell_atoms[p], rank is the inverse. A system's positions are [begin, begin + natoms),
+  // like its atoms. The pair phase (Verlet and neighbor rows, charge matrix, charge solve, non-bonded pairs) works in
+  // this order: row p is the row of atom cell_atoms[p] and its entries name partners by position, so the entries of a
+  // run of consecutive cells name consecutive positions and a warp's gathers fall into few cache lines.
   int* cell_atoms;       // atoms sorted by cell
+  int* rank;             // atom -> position in cell order
+  double4* xr;           // current positions in cell order; w packs (type, atom): ord_type, ord_atom
+  double* qr;            // charges in cell order
   float4* xs;            // positions in cell order relative to their system's origin, single precision (w = type)
   int* cell_start;       // ncell_total + 1
   int ncell_total;
@@ -211,6 +218,12 @@ __device__ inline void pair_dvec_x(const Dev& d, const SysInfo& s, int i, int j,
 __device__ inline void pair_dvec(const Dev& d, const SysInfo& s, int i, int j, int sidx, double* dv) {
   pair_dvec_x(d, s, i, j, sidx, d.x[i], d.x[j], dv);
 }
+
+__device__ inline double4 ord_pack(const double4& x, int type, int atom) {
+  return make_double4(x.x, x.y, x.z, __hiloint2double(type, atom));
+}
+__device__ inline int ord_type(const double4& xr) { return __double2hiint(xr.w); }
+__device__ inline int ord_atom(const double4& xr) { return __double2loint(xr.w); }
 
 // A list of this evaluation overflowed (the host grows it and repeats the evaluation): later kernels skip their work.
 __device__ inline bool lists_failed(const Dev& d) {

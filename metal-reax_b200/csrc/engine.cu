@@ -118,8 +118,10 @@ struct Context {
   std::vector<int> htype;
   std::vector<SysInfo> huser;   // systems as the caller gave them
   DBuf<SysInfo> sys;
-  DBuf<int> sys_of, type, cell_key, cell_key_sorted, cell_atoms, atom_iota, cell_start, sys_flag;
+  DBuf<int> sys_of, type, cell_key, cell_key_sorted, cell_atoms, rank, atom_iota, cell_start, sys_flag;
   DBuf<float4> xs;
+  DBuf<double4> xr;
+  DBuf<double> qr;
   DBuf<long long> tag;
   DBuf<double4> x;
   DBuf<double> q;
@@ -152,7 +154,7 @@ struct Context {
   DBuf<double> epart;   // per (system, 256-atom chunk) partial sums of the energy terms and virial components
   int echunks = 1;
   // QEq
-  DBuf<double2> cg_x, cg_b, cg_r, cg_d, cg_p, cg_q;
+  DBuf<double2> cg_x, cg_b, cg_r, cg_d, cg_p, cg_q, cg_s;
   DBuf<float2> cg_df;
   DBuf<double> cg_eta, cg_part, s_hist, t_hist, cg_rel;
   DBuf<int> cg_iters, cg_nlive, cg_nref, cg_brk;
@@ -578,13 +580,18 @@ struct Context {
     cell_key.ensure(static_cast<size_t>(na));
     cell_key_sorted.ensure(static_cast<size_t>(na));
     cell_atoms.ensure(static_cast<size_t>(na));
+    rank.ensure(static_cast<size_t>(na));
     xs.ensure(static_cast<size_t>(na));
+    xr.ensure(static_cast<size_t>(na));
+    qr.ensure(static_cast<size_t>(na));
     atom_iota.ensure(static_cast<size_t>(na));
     cell_start.ensure(static_cast<size_t>(ncell_total) + 1);
     {
       std::vector<int> io(static_cast<size_t>(na));
       for (int a = 0; a < na; ++a) io[static_cast<size_t>(a)] = a;
       RXCU(cudaMemcpy(atom_iota.p, io.data(), sizeof(int) * na, cudaMemcpyHostToDevice));
+      // until the first rebuild (which every evaluation of a new layout starts with) the cell order is the atom order
+      RXCU(cudaMemcpy(rank.p, atom_iota.p, sizeof(int) * na, cudaMemcpyDeviceToDevice));
     }
     key_bits = 1;
     while ((1LL << key_bits) <= ncell_total) ++key_bits;
@@ -627,7 +634,7 @@ struct Context {
     vir.ensure(n * kVir);
     vir_nb.ensure(n * kVir); vir_h.ensure(n * kVir); vir_t.ensure(n * kVir);
     fown_h.ensure(n); fown_t.ensure(n); fix_h.ensure(3 * n); pe_fix.ensure(n);
-    cg_x.ensure(n); cg_df.ensure(n); cg_b.ensure(n); cg_r.ensure(n); cg_d.ensure(n); cg_p.ensure(n); cg_q.ensure(n); cg_eta.ensure(n);
+    cg_x.ensure(n); cg_df.ensure(n); cg_b.ensure(n); cg_r.ensure(n); cg_d.ensure(n); cg_p.ensure(n); cg_q.ensure(n); cg_s.ensure(n); cg_eta.ensure(n);
     cg_iters.ensure(2 * static_cast<size_t>(nsys)); cg_rel.ensure(2 * static_cast<size_t>(nsys));
     cg_sys.ensure(nsys); cg_rb0.ensure(n); cg_rb1.ensure(n); cg_nlive.ensure(2);
     cg_part.ensure(16 * static_cast<size_t>(std::max(nsm, 1)) * 32);
@@ -659,7 +666,7 @@ struct Context {
   Dev dev() {
     Dev d{};
     d.na = na; d.nsys = nsys; d.sys = sys.p; d.sys_of = sys_of.p; d.x = x.p; d.type = type.p; d.tag = tag.p; d.q = q.p;
-    d.cell_key = cell_key.p; d.cell_atoms = cell_atoms.p; d.xs = xs.p; d.cell_start = cell_start.p; d.ncell_total = ncell_total;
+    d.cell_key = cell_key.p; d.cell_atoms = cell_atoms.p; d.rank = rank.p; d.xr = xr.p; d.qr = qr.p; d.xs = xs.p; d.cell_start = cell_start.p; d.ncell_total = ncell_total;
     d.ncap = ncap; d.nbr = nbr.p; d.nbr_cnt = nbr_cnt.p; d.hhi = hhi.p; d.hlo = hlo.p;
     d.vcap = vcap; d.vrow = vrow.p; d.vcnt = vcnt.p; d.xref = xref.p; d.sys_flag = sys_flag.p;
     d.rv2 = (ff.nonb_cut + skin) * (ff.nonb_cut + skin);
@@ -777,7 +784,7 @@ struct Context {
   CgArgs cg_args() {
     CgArgs a{};
     a.imax = qeq_imax; a.tol = qeq_tol;
-    a.x = cg_x.p; a.b = cg_b.p; a.r = cg_r.p; a.d = cg_d.p; a.p = cg_p.p; a.q = cg_q.p; a.df = cg_df.p; a.eta = cg_eta.p; a.part = cg_part.p;
+    a.x = cg_x.p; a.b = cg_b.p; a.r = cg_r.p; a.d = cg_d.p; a.p = cg_p.p; a.q = cg_q.p; a.s = cg_s.p; a.df = cg_df.p; a.eta = cg_eta.p; a.part = cg_part.p;
     a.out_iters = cg_iters.p; a.out_rel = cg_rel.p; a.out_nref = cg_nref.p; a.out_brk = cg_brk.p; a.write_q = 1;
     return a;
   }
@@ -796,18 +803,27 @@ struct Context {
     int cg_per_sm = 2;
   } tune;
   int grid_occ[5] = {0, 0, 0, 0, 0}, seg_per_sm = 0;
+  static constexpr int kCgSmem = 220 * 1024;   // dynamic shared memory of the single-system CG at most
   void launch_cg(const Dev& d, CgArgs a) {
     if (nsys == 1 && na > tune.lone_grid_min) {   // one large system: all SMs on its rows, block partials in block order
       const int units = tune.cg_per_sm > 0 ? std::min(tune.cg_per_sm, 4) : 4;
       const int threads = 256 * units;
-      if (!grid_occ[units]) RXCU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&grid_occ[units], k_cg_grid, threads, 0));
-      if (grid_occ[units] < 1) throw Error(RX_ERR_CUDA, "the single-system CG block does not fit on an SM");
       int grid = std::max(1, std::min(nsm, (na + (threads / 32) - 1) / (threads / 32)));
+      // the rows' vectors and lengths in shared memory where they fit beside the rings (108 bytes a row)
+      const int rows = (na + grid - 1) / grid;
+      const size_t rings = static_cast<size_t>(threads / 32) * kRingBytes, with_rows = rings + 108 * static_cast<size_t>(rows);
+      a.smem_rows = with_rows <= kCgSmem ? rows : 0;
+      const size_t smem = a.smem_rows ? with_rows : rings;
+      if (!grid_occ[units]) {
+        RXCU(cudaFuncSetAttribute(k_cg_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgSmem));
+        RXCU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&grid_occ[units], k_cg_grid, threads, kCgSmem));
+      }
+      if (grid_occ[units] < 1) throw Error(RX_ERR_CUDA, "the single-system CG block does not fit on an SM");
       a.begin = 0;
       a.n = na;
       void* args[] = {const_cast<Dev*>(&d), &a};
       ++launches;
-      RXCU(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_cg_grid), dim3(grid), dim3(threads), args, 0, stream));
+      RXCU(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_cg_grid), dim3(grid), dim3(threads), args, smem, stream));
     } else {   // a batch (or one small system): every row of every system on all SMs, per-system fixed-order sums
       const int threads = 256;
       if (!seg_per_sm) RXCU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&seg_per_sm, k_cg_seg, threads, 0));
@@ -1224,6 +1240,10 @@ struct Context {
         RXCU(cudaMemcpyAsync(g_out, xyz3.p, sizeof(double) * 3 * na, cudaMemcpyDeviceToHost, gs));
       }
       energy_sums();
+      if ((cen_out || counts) && !pe_on) {   // k_nonbonded_half does not count
+        ++launches;
+        k_count_pairs<<<blocks(static_cast<long long>(na) * 32, 128), 128, 0, stream>>>(dev());
+      }
       if (e_out) {
         eh = energy_stage(static_cast<size_t>(kTerms) * nsys);
         RXCU(cudaMemcpyAsync(eh, energies.p, sizeof(double) * kTerms * nsys, cudaMemcpyDeviceToHost, stream));
@@ -1408,7 +1428,9 @@ struct Context {
     fetch_qeq_counts();
     std::vector<double2> xh(static_cast<size_t>(na));
     std::vector<int> brk(static_cast<size_t>(nsys));
-    RXCU(cudaMemcpyAsync(xh.data(), cg_x.p, sizeof(double2) * na, cudaMemcpyDeviceToHost, stream));
+    ++launches;
+    k_to_atom_order<<<blocks(na, 256), 256, 0, stream>>>(d, cg_x.p, cg_p.p);
+    RXCU(cudaMemcpyAsync(xh.data(), cg_p.p, sizeof(double2) * na, cudaMemcpyDeviceToHost, stream));
     RXCU(cudaMemcpyAsync(brk.data(), cg_brk.p, sizeof(int) * nsys, cudaMemcpyDeviceToHost, stream));
     RXCU(cudaStreamSynchronize(stream));
     RXCU(cudaGetLastError());
@@ -1447,8 +1469,9 @@ struct Context {
     rows_only();
     std::vector<double2> h(static_cast<size_t>(na));
     for (int a = 0; a < na; ++a) h[static_cast<size_t>(a)] = make_double2(vin[a], 0.0);
-    RXCU(cudaMemcpyAsync(cg_d.p, h.data(), sizeof(double2) * na, cudaMemcpyHostToDevice, stream));
-    ++launches;
+    RXCU(cudaMemcpyAsync(cg_p.p, h.data(), sizeof(double2) * na, cudaMemcpyHostToDevice, stream));
+    launches += 2;
+    k_to_cell_order<<<blocks(na, 256), 256, 0, stream>>>(dev(), cg_p.p, cg_d.p);
     k_qeq_matvec<<<blocks(static_cast<long long>(na) * 32, 128), 128, 0, stream>>>(dev(), dff, cg_d.p, cg_q.p);
     RXCU(cudaMemcpyAsync(h.data(), cg_q.p, sizeof(double2) * na, cudaMemcpyDeviceToHost, stream));
     RXCU(cudaStreamSynchronize(stream));

@@ -20,6 +20,8 @@ struct SysCg {
   unsigned counter;   // rows of this system that have arrived in the current pass
 };
 
+constexpr int kRingBytes = 6144;   // shared memory per warp of the charge solve's row products (rows_stream)
+
 struct CgArgs {
   int begin, n, imax;
   double tol;
@@ -29,7 +31,9 @@ struct CgArgs {
   double2* d;
   double2* p;
   double2* q;
-  float2* df;     // FP32 copy of d, gathered by the single-precision-matrix iterations (single-system CG)
+  double2* s;      // A d (single-system CG)
+  float2* df;      // FP32 copy of M^-1 r, gathered by the single-precision-matrix iterations (single-system CG)
+  int smem_rows;   // rows per block whose vectors fit its shared memory (single-system CG; 0: vectors in global memory)
   double* eta;
   double* part;    // 2 * 8 * gridDim.x partial sums (double-buffered)
   int* out_iters;
@@ -52,6 +56,7 @@ __global__ void k_neighbors(Dev d, DevFF ff);
 __global__ void k_pairs(Dev d, DevFF ff, QeqParams qp);
 __global__ void k_nonbonded(Dev d, DevFF ff);
 __global__ void k_nonbonded_half(Dev d, DevFF ff);
+__global__ void k_count_pairs(Dev d);
 __global__ void k_acks2(Dev d, DevFF ff, const double* s_kin);
 __global__ void k_cg_grid(Dev d, CgArgs a);
 __global__ void k_cg_seg(Dev d, CgArgs a);
@@ -59,6 +64,8 @@ __global__ void k_qeq_prepare(Dev d, DevFF ff, CgArgs a, const double* s_hist, c
 __global__ void k_qeq_prepare_given(Dev d, DevFF ff, CgArgs a, const double* b, const double* x0);
 __global__ void k_qeq_history(Dev d, const double2* x, double* s_hist, double* t_hist, int strict);
 __global__ void k_qeq_matvec(Dev d, DevFF ff, const double2* v, double2* y);
+__global__ void k_to_cell_order(Dev d, const double2* by_atom, double2* by_position);
+__global__ void k_to_atom_order(Dev d, const double2* by_position, double2* by_atom);
 __global__ void k_energy_part(Dev d, double* part, int nchunk);
 __global__ void k_energy_final(Dev d, const double* part, int nchunk, double* out, double* out_vir);
 

@@ -1,6 +1,8 @@
 // Cell lists, full neighbor rows with the charge matrix, non-bonded forces, charge-equilibration CG, energy sums.
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "device.cuh"
 #include "kernels.hpp"
 
@@ -19,7 +21,11 @@ __global__ void k_nbr_check(Dev d) {
   for (int c = 0; c < 3; ++c) d.fix_h[3 * static_cast<size_t>(a) + c] = 0ull;
   if (d.pe_on) d.pe_fix[a] = 0ull;
   const int s = d.sys_of[a];
+  const int p = d.rank[a], ta = d.type[a];
   const double4 x = d.x[a];
+  // the cell-ordered copies of the pair phase (a rebuild, which changes the order, writes them again: k_cell_start)
+  d.xr[p] = ord_pack(x, ta, a);
+  d.qr[p] = d.q[a];
   if (!(isfinite(x.x) && isfinite(x.y) && isfinite(x.z))) {
     atomicOr(d.status, ST_NONFINITE);
     return;
@@ -42,6 +48,7 @@ __global__ void k_nbr_check(Dev d) {
       y.y -= n[0] * sy.L[1] + n[1] * sy.L[4] + n[2] * sy.L[7];
       y.z -= n[0] * sy.L[2] + n[1] * sy.L[5] + n[2] * sy.L[8];
       d.x[a] = y;
+      d.xr[p] = ord_pack(y, ta, a);
       dx = y.x - r.x; dy = y.y - r.y; dz = y.z - r.z;
     }
   }
@@ -104,8 +111,9 @@ __global__ void k_rebuild_flag(Dev d, cudaGraphConditionalHandle h) {
   if (threadIdx.x == 0) cudaGraphSetConditional(h, any ? 1u : 0u);
 }
 
-// cell_start[c] = first position in the sorted order whose key is >= c; positions gathered into cell order, relative to
-// their system's origin and rounded to single precision (the candidate scan of the Verlet rows reads only these)
+// cell_start[c] = first position in the sorted order whose key is >= c; the atoms' ranks and cell-ordered positions and
+// charges; and positions relative to their system's origin and rounded to single precision (the candidate scan of the
+// Verlet rows reads only these)
 __global__ void k_cell_start(Dev d, const int* sorted_keys) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p > d.na) return;
@@ -115,6 +123,9 @@ __global__ void k_cell_start(Dev d, const int* sorted_keys) {
   if (p < d.na) {
     const int a = d.cell_atoms[p];
     const double4 x = d.x[a];
+    d.rank[a] = p;
+    d.xr[p] = ord_pack(x, d.type[a], a);
+    d.qr[p] = d.q[a];
     const double* o = d.sys[d.sys_of[a]].origin;
     d.xs[p] = make_float4(static_cast<float>(x.x - o[0]), static_cast<float>(x.y - o[1]), static_cast<float>(x.z - o[2]),
                           static_cast<float>(d.type[a]));
@@ -132,7 +143,7 @@ __device__ inline void taper_horner(const double* c, double r, double& Tap, doub
   dTap = g;
 }
 
-// Verlet rows, one warp per atom of a system being rebuilt: every image within nonb_cut + skin (a superset of the
+// Verlet rows (in cell order, entries by cell-order position), one warp per atom of a system being rebuilt: every image within nonb_cut + skin (a superset of the
 // owned-row cut-off of build_far_list, src/neighbor/neighbor.cpp:180-212). The cells within `range` of the atom's cell
 // are visited as runs of consecutive cells along x (one contiguous range of the cell-ordered atoms per run and periodic
 // image), so the candidate loads are coalesced. Entries are written through a warp ballot in visiting order
@@ -144,7 +155,7 @@ __global__ void __launch_bounds__(128, 6) k_neighbors(Dev d, DevFF ff) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= d.na) return;
-  const int i = warp;
+  const int pi = warp, i = d.cell_atoms[warp];
   const int sy = d.sys_of[i];
   if (!d.sys_flag[sy]) return;
   const SysInfo& s = d.sys[sy];
@@ -155,7 +166,7 @@ __global__ void __launch_bounds__(128, 6) k_neighbors(Dev d, DevFF ff) {
   int count = 0, count_near = 0, count_acc = 0;
   const unsigned lt = (1u << lane) - 1u;
   const int center = (d.S * d.S * d.S - 1) / 2;
-  const size_t rowbase = static_cast<size_t>(i) * d.vcap;
+  const size_t rowbase = static_cast<size_t>(pi) * d.vcap;
   const bool hb_i = static_cast<int>(ff.sb[d.type[i] * SB_N + SB_P_HBOND]) == 1;
   const float tv = s.vthr[0], tn = s.vthr[1], ta = s.vthr[2];
   const int smax = d.smax, S = d.S, sbase = s.shift_base;
@@ -218,17 +229,18 @@ __global__ void __launch_bounds__(128, 6) k_neighbors(Dev d, DevFF ff) {
             j = d.cell_atoms[p];
             const float4 xj = d.xs[p];
             tj = xj.w;
-            if (!(j == i && sidx == center)) {
+            if (!(p == pi && sidx == center)) {
               const float dx = xj.x + cimg.x, dy = xj.y + cimg.y, dz = xj.z + cimg.z;
               r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
               ok = r2 <= tv;
             }
           }
-          const unsigned code = static_cast<unsigned>(j) | (static_cast<unsigned>(sidx) << d.abits);
+          const unsigned image = static_cast<unsigned>(sidx) << d.abits;
+          const unsigned code = static_cast<unsigned>(j) | image;   // the bonded chain's rows name atoms
           const unsigned m = __ballot_sync(0xffffffffu, ok);
           if (ok) {
             const int pos = count + __popc(m & lt);
-            if (pos < d.vcap) d.vrow[rowbase + pos] = code;
+            if (pos < d.vcap) d.vrow[rowbase + pos] = static_cast<unsigned>(p) | image;
           }
           count += __popc(m);
           // the short Verlet rows of the bond and H-bond kernels (their own exact tests run on every evaluation)
@@ -253,7 +265,7 @@ __global__ void __launch_bounds__(128, 6) k_neighbors(Dev d, DevFF ff) {
     }
   }
   if (lane == 0) {
-    d.vcnt[i] = count;
+    d.vcnt[pi] = count;
     if (count > d.vcap) {
       atomicOr(d.status, ST_VERLET_OVERFLOW);
       atomicMax(d.status + 4, count);
@@ -282,27 +294,27 @@ __global__ void __launch_bounds__(256) k_pairs(Dev d, DevFF ff, QeqParams qp) {
   const int lane = threadIdx.x & 31;
   if (warp >= d.na) return;
   if (lists_failed(d)) return;
-  const int i = warp;
-  const SysInfo s = d.sys[d.sys_of[i]];
+  const SysInfo s = d.sys[d.sys_of[warp]];
   const double rc2 = ff.nonb_cut * ff.nonb_cut;
-  const double4 xi = d.x[i];
-  const int ti = d.type[i];
+  const double4 xi = d.xr[warp];
+  const int ti = ord_type(xi), i = ord_atom(xi);
   const double* shld_i = ff.shld + static_cast<size_t>(ti) * ff.nt;
   int count = 0;
   const unsigned lt = (1u << lane) - 1u;
-  const size_t vbase = static_cast<size_t>(i) * d.vcap, rowbase = static_cast<size_t>(i) * d.ncap;
-  const int nv = min(d.vcnt[i], d.vcap);
+  const size_t vbase = static_cast<size_t>(warp) * d.vcap, rowbase = static_cast<size_t>(warp) * d.ncap;
+  const int nv = min(d.vcnt[warp], d.vcap);
   for (int base = 0; base < nv; base += 32) {
     const int e = base + lane;
     bool ok = false;
     unsigned code = 0;
-    int j = 0;
+    int tj = 0;
     double r2 = 0.0;
     if (e < nv) {
       code = d.vrow[vbase + e];
-      j = static_cast<int>(code & d.amask);
+      const double4 xj = d.xr[code & d.amask];
+      tj = ord_type(xj);
       double dv[3];
-      pair_dvec_x(d, s, i, j, static_cast<int>(code >> d.abits), xi, d.x[j], dv);
+      pair_dvec_x(d, s, i, ord_atom(xj), static_cast<int>(code >> d.abits), xi, xj, dv);
       r2 = dv[0] * dv[0] + dv[1] * dv[1] + dv[2] * dv[2];
       ok = r2 <= rc2;
     }
@@ -316,7 +328,7 @@ __global__ void __launch_bounds__(256) k_pairs(Dev d, DevFF ff, QeqParams qp) {
         if (r <= qp.swb) {
           double Tap, dTap;
           taper_horner(qp.tap, r, Tap, dTap);
-          const double a3 = r * r * r + shld_i[d.type[j]];
+          const double a3 = r * r * r + shld_i[tj];
           // z = a3^(-1/3): single-precision seed, then two Newton steps z <- z + (z/3)(1 - a3 z^3), which
           // square the relative error each (1e-7 -> 1e-14 -> rounding level); no division
           double z = static_cast<double>(rcbrtf(static_cast<float>(a3)));
@@ -331,7 +343,7 @@ __global__ void __launch_bounds__(256) k_pairs(Dev d, DevFF ff, QeqParams qp) {
     count += __popc(m);
   }
   if (lane == 0) {
-    d.nbr_cnt[i] = count;
+    d.nbr_cnt[warp] = min(count, d.ncap);
     if (count > d.ncap) {
       atomicOr(d.status, ST_NBR_OVERFLOW);
       atomicMax(d.status + 1, count);
@@ -396,7 +408,7 @@ __device__ __forceinline__ float nb_pair_terms(const DevFF& ff, int ti, int tj, 
     }
   }
   const float z = rcbrtf(r2f * r + pp[7]);
-  const float cq = 332.06371f * qi * qj;
+  const float cq = 332.06371f * (qi * qj);   // the same bits from both ends of the pair
   e_ele = cq * (Tap * z);
   const float CEclmb = cq * (dTap - Tap * r * (z * z * z)) * z;
   return CEvd + CEclmb;
@@ -412,28 +424,29 @@ __global__ void k_nonbonded(Dev d, DevFF ff) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= d.na) return;
-  const int i = warp;
-  const SysInfo s = d.sys[d.sys_of[i]];
-  const int ti = d.type[i];
-  const int cnt = min(d.nbr_cnt[i], d.ncap);
+  const SysInfo s = d.sys[d.sys_of[warp]];
+  const double4 xi4 = d.xr[warp];
+  const int ti = ord_type(xi4), i = ord_atom(xi4);
+  const int cnt = d.nbr_cnt[warp];
   const float p_vdW1 = static_cast<float>(ff.gp[28]), p_vdW1i = 1.f / p_vdW1;
   const float swa = static_cast<float>(ff.nonb_low), inv_dd = static_cast<float>(1.0 / (ff.nonb_cut - ff.nonb_low));
-  const float qi = static_cast<float>(d.q[i]);
+  const double qd = d.qr[warp];
+  const float qi = static_cast<float>(qd);
   const long long tag_i = d.tag[i];
   const int center = (d.S * d.S * d.S - 1) / 2;
   double gx = 0, gy = 0, gz = 0, ev = 0, ee = 0, ehalf = 0;
   float v0 = 0, v1 = 0, v2 = 0, v3 = 0, v4 = 0, v5 = 0;   // pair virial, half per directed entry (lane partials)
   int counted = 0;
-  const double4 xi4 = d.x[i];
   for (int e = lane; e < cnt; e += 32) {
-    const unsigned code = d.nbr[static_cast<size_t>(i) * d.ncap + e];
-    const int j = static_cast<int>(code & d.amask);
+    const unsigned code = d.nbr[static_cast<size_t>(warp) * d.ncap + e];
+    const int pj = static_cast<int>(code & d.amask);
     const int sidx = static_cast<int>(code >> d.abits);
+    const double4 xj = d.xr[pj];
+    const int j = ord_atom(xj);
     double dvd[3];
-    pair_dvec_x(d, s, i, j, sidx, xi4, d.x[j], dvd);
-    const int tj = d.type[j];
+    pair_dvec_x(d, s, i, j, sidx, xi4, xj, dvd);
     float e_vdW, e_ele;
-    const float CE = nb_pair_terms(ff, ti, tj, qi, static_cast<float>(d.q[j]), dvd, p_vdW1, p_vdW1i, swa, inv_dd, e_vdW, e_ele);
+    const float CE = nb_pair_terms(ff, ti, ord_type(xj), qi, static_cast<float>(d.qr[pj]), dvd, p_vdW1, p_vdW1i, swa, inv_dd, e_vdW, e_ele);
     const float dx = static_cast<float>(dvd[0]), dy = static_cast<float>(dvd[1]), dz = static_cast<float>(dvd[2]);
     gx -= static_cast<double>(CE * dx);
     gy -= static_cast<double>(CE * dy);
@@ -476,17 +489,19 @@ __global__ void k_nonbonded(Dev d, DevFF ff) {
     vi[0] = w0; vi[1] = w1; vi[2] = w2; vi[3] = w3; vi[4] = w4; vi[5] = w5;
     d.eatom[static_cast<size_t>(i) * kTerms + E_VDW] = ev;
     d.eatom[static_cast<size_t>(i) * kTerms + E_ELE] = ee;
-    const double chi = ff.sb[ti * SB_N + SB_CHI], eta = ff.sb[ti * SB_N + SB_ETA], qd = d.q[i];
+    const double chi = ff.sb[ti * SB_N + SB_CHI], eta = ff.sb[ti * SB_N + SB_ETA];
     d.eatom[static_cast<size_t>(i) * kTerms + E_POL] = 23.02 * (chi * qd + (eta / 2.) * (qd * qd));
     if (d.pe_on) pe_add(d, i, ehalf + 23.02 * (chi * qd + (eta / 2.) * (qd * qd)));
     d.census[4 * d.na + i] = counted;
   }
 }
 
-// Each non-bonded pair once: the same terms as k_nonbonded over the counted entries of every row only (the
-// owner-computes rule above picks exactly one entry of each pair), with the partner's gradient +CE dv added to its
-// fixed-point accumulator (2^32 units: integer additions give the same sum in any order, so the result is
-// deterministic). The counted entries of a row are gathered into a per-warp queue in row order, so every lane of a
+// Each non-bonded pair once: the same terms as k_nonbonded over one entry of every pair, with the partner's gradient +CE dv
+// added to its fixed-point accumulator (2^32 units: integer additions give the same sum in any order, so the result is
+// deterministic). The entry taken is the one whose partner stands later in cell order (for an image of the atom itself,
+// the one with the larger shift index): read off the code alone, where the reference's owner rule
+// (classify_nonbonded_entry) would need the atoms' numbers and tags. The sums are over the same pairs; the census of
+// that rule is k_count_pairs. The entries taken are gathered into a per-warp queue in row order, so every lane of a
 // batch of 32 has a pair to compute. The pair virial goes whole to the owner; the per-atom split of energies and
 // virials (RX_COMPUTE_PERATOM) takes k_nonbonded instead.
 __global__ void __launch_bounds__(256) k_nonbonded_half(Dev d, DevFF ff) {
@@ -495,42 +510,40 @@ __global__ void __launch_bounds__(256) k_nonbonded_half(Dev d, DevFF ff) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
   if (warp >= d.na) return;
-  const int i = warp;
-  const SysInfo s = d.sys[d.sys_of[i]];
-  const int ti = d.type[i];
-  const int cnt = min(d.nbr_cnt[i], d.ncap);
+  const SysInfo s = d.sys[d.sys_of[warp]];
+  const double4 xi4 = d.xr[warp];
+  const int ti = ord_type(xi4), i = ord_atom(xi4);
+  const int cnt = d.nbr_cnt[warp];
   const float p_vdW1 = static_cast<float>(ff.gp[28]), p_vdW1i = 1.f / p_vdW1;
   const float swa = static_cast<float>(ff.nonb_low), inv_dd = static_cast<float>(1.0 / (ff.nonb_cut - ff.nonb_low));
-  const float qi = static_cast<float>(d.q[i]);
-  const long long tag_i = d.tag[i];
+  const double qd = d.qr[warp];
+  const float qi = static_cast<float>(qd);
   const int center = (d.S * d.S * d.S - 1) / 2;
   const unsigned lt = (1u << lane) - 1u;
   double gx = 0, gy = 0, gz = 0, ev = 0, ee = 0;
   float v0 = 0, v1 = 0, v2 = 0, v3 = 0, v4 = 0, v5 = 0;   // pair virials (lane partials)
-  int counted = 0;
-  const double4 xi4 = d.x[i];
   auto pair = [&](unsigned code) {
-    const int j = static_cast<int>(code & d.amask);
-    const int sidx = static_cast<int>(code >> d.abits);
+    const int pj = static_cast<int>(code & d.amask);
+    const double4 xj = d.xr[pj];
     double dvd[3];
-    pair_dvec_x(d, s, i, j, sidx, xi4, d.x[j], dvd);
+    pair_dvec_x(d, s, i, ord_atom(xj), static_cast<int>(code >> d.abits), xi4, xj, dvd);
     float e_vdW, e_ele;
-    const float CE = nb_pair_terms(ff, ti, d.type[j], qi, static_cast<float>(d.q[j]), dvd, p_vdW1, p_vdW1i, swa, inv_dd,
+    const float CE = nb_pair_terms(ff, ti, ord_type(xj), qi, static_cast<float>(d.qr[pj]), dvd, p_vdW1, p_vdW1i, swa, inv_dd,
                                    e_vdW, e_ele);
     const float dx = static_cast<float>(dvd[0]), dy = static_cast<float>(dvd[1]), dz = static_cast<float>(dvd[2]);
     const float fx = CE * dx, fy = CE * dy, fz = CE * dz;
     gx -= static_cast<double>(fx);
     gy -= static_cast<double>(fy);
     gz -= static_cast<double>(fz);
-    fix_add(d.fix_h + 3 * static_cast<size_t>(j), static_cast<double>(fx));
-    fix_add(d.fix_h + 3 * static_cast<size_t>(j) + 1, static_cast<double>(fy));
-    fix_add(d.fix_h + 3 * static_cast<size_t>(j) + 2, static_cast<double>(fz));
+    unsigned long long* fj = d.fix_h + 3 * static_cast<size_t>(ord_atom(xj));
+    fix_add(fj, static_cast<double>(fx));
+    fix_add(fj + 1, static_cast<double>(fy));
+    fix_add(fj + 2, static_cast<double>(fz));
     const float c = -CE;   // the pair virial -CE dv (x) dv, whole
     v0 += c * dx * dx; v1 += c * dy * dy; v2 += c * dz * dz;
     v3 += c * dx * dy; v4 += c * dx * dz; v5 += c * dy * dz;
     ev += static_cast<double>(e_vdW);
     ee += static_cast<double>(e_ele);
-    ++counted;
   };
   int qn = 0;   // entries waiting in this warp's queue (warp-uniform)
   for (int base = 0; base < cnt; base += 32) {
@@ -538,26 +551,10 @@ __global__ void __launch_bounds__(256) k_nonbonded_half(Dev d, DevFF ff) {
     bool own = false;
     unsigned code = 0;
     if (e < cnt) {
-      code = d.nbr[static_cast<size_t>(i) * d.ncap + e];
-      const int j = static_cast<int>(code & d.amask);
+      code = d.nbr[static_cast<size_t>(warp) * d.ncap + e];
+      const int pj = static_cast<int>(code & d.amask);
       const int sidx = static_cast<int>(code >> d.abits);
-      if (sidx == center) {
-        own = j > i;
-      } else {
-        const long long tag_j = d.tag[j];
-        if (tag_i < tag_j) {
-          own = true;
-        } else if (tag_i == tag_j) {   // an image of i itself: the positive direction
-          double dvd[3];
-          pair_dvec_x(d, s, i, j, sidx, xi4, d.x[j], dvd);
-          const double SMALL = 1e-4;
-          if (dvd[2] > SMALL) own = true;
-          else if (fabs(dvd[2]) < SMALL) {
-            if (dvd[1] > SMALL) own = true;
-            else if (fabs(dvd[1]) < SMALL && dvd[0] > SMALL) own = true;
-          }
-        }
-      }
+      own = pj > warp || (pj == warp && sidx > center);
     }
     const unsigned m = __ballot_sync(0xffffffffu, own);
     if (own) queue[wb][qn + __popc(m & lt)] = code;
@@ -574,20 +571,55 @@ __global__ void __launch_bounds__(256) k_nonbonded_half(Dev d, DevFF ff) {
     }
   }
   if (lane < qn) pair(queue[wb][lane]);
-  gx = warp_sum(gx); gy = warp_sum(gy); gz = warp_sum(gz); ev = warp_sum(ev); ee = warp_sum(ee);
-  const double w0 = warp_sum(static_cast<double>(v0)), w1 = warp_sum(static_cast<double>(v1)), w2 = warp_sum(static_cast<double>(v2));
-  const double w3 = warp_sum(static_cast<double>(v3)), w4 = warp_sum(static_cast<double>(v4)), w5 = warp_sum(static_cast<double>(v5));
-  for (int o = 16; o > 0; o >>= 1) counted += __shfl_xor_sync(0xffffffffu, counted, o);
-  if (lane == 0) {
-    d.fnb[i] = make_double4(gx, gy, gz, 0.0);
-    double* vi = d.vir_nb + static_cast<size_t>(i) * kVir;
-    vi[0] = w0; vi[1] = w1; vi[2] = w2; vi[3] = w3; vi[4] = w4; vi[5] = w5;
-    d.eatom[static_cast<size_t>(i) * kTerms + E_VDW] = ev;
-    d.eatom[static_cast<size_t>(i) * kTerms + E_ELE] = ee;
-    const double chi = ff.sb[ti * SB_N + SB_CHI], eta = ff.sb[ti * SB_N + SB_ETA], qd = d.q[i];
-    d.eatom[static_cast<size_t>(i) * kTerms + E_POL] = 23.02 * (chi * qd + (eta / 2.) * (qd * qd));
-    d.census[4 * d.na + i] = counted;
+  double sums[16] = {gx, gy, gz, ev, ee, v0, v1, v2, v3, v4, v5, 0, 0, 0, 0, 0};
+  const double total = warp_sums<16>(sums);
+  if ((lane & 1) == 0) {   // lane 2 k holds sum k
+    const int k = lane >> 1;
+    double* ea = d.eatom + static_cast<size_t>(i) * kTerms;
+    if (k < 3) reinterpret_cast<double*>(d.fnb + i)[k] = total;
+    else if (k == 3) ea[E_VDW] = total;
+    else if (k == 4) ea[E_ELE] = total;
+    else if (k < 11) d.vir_nb[static_cast<size_t>(i) * kVir + k - 5] = total;
+    else if (k == 11) {
+      const double chi = ff.sb[ti * SB_N + SB_CHI], eta = ff.sb[ti * SB_N + SB_ETA];
+      ea[E_POL] = 23.02 * (chi * qd + (eta / 2.) * (qd * qd));
+    }
   }
+}
+
+// The counted non-bonded pairs of every atom (owner-computes rule, classify_nonbonded_entry,
+// src/neighbor/neighbor.cpp:295-310, as in k_nonbonded) for the decision census
+__global__ void k_count_pairs(Dev d) {
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (warp >= d.na) return;
+  const SysInfo s = d.sys[d.sys_of[warp]];
+  const double4 xi = d.xr[warp];
+  const int i = ord_atom(xi), cnt = d.nbr_cnt[warp];
+  const long long tag_i = d.tag[i];
+  const int center = (d.S * d.S * d.S - 1) / 2;
+  int counted = 0;
+  for (int e = lane; e < cnt; e += 32) {
+    const unsigned code = d.nbr[static_cast<size_t>(warp) * d.ncap + e];
+    const int sidx = static_cast<int>(code >> d.abits);
+    const double4 xj = d.xr[code & d.amask];
+    const int j = ord_atom(xj);
+    if (sidx == center) {
+      counted += j > i;
+      continue;
+    }
+    const long long tag_j = d.tag[j];
+    if (tag_i != tag_j) {
+      counted += tag_i < tag_j;
+      continue;
+    }
+    double dv[3];   // an image of i itself: the positive direction
+    pair_dvec_x(d, s, i, j, sidx, xi, xj, dv);
+    const double SMALL = 1e-4;
+    counted += dv[2] > SMALL || (fabs(dv[2]) < SMALL && (dv[1] > SMALL || (fabs(dv[1]) < SMALL && dv[0] > SMALL)));
+  }
+  for (int o = 16; o > 0; o >>= 1) counted += __shfl_xor_sync(0xffffffffu, counted, o);
+  if (lane == 0) d.census[4 * d.na + i] = counted;
 }
 
 // ------------------------------------------------------------------------------------------------ ACKS2 pair terms
@@ -602,22 +634,23 @@ __global__ void k_acks2(Dev d, DevFF ff, const double* s_kin) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= d.na) return;
-  const int i = warp;
-  const SysInfo s = d.sys[d.sys_of[i]];
-  const int ti = d.type[i];
-  const int cnt = min(d.nbr_cnt[i], d.ncap);
+  const SysInfo s = d.sys[d.sys_of[warp]];
+  const double4 xi4 = d.xr[warp];
+  const int ti = ord_type(xi4), i = ord_atom(xi4);
+  const int cnt = d.nbr_cnt[warp];
   const double softness = ff.gp[34];
   const double bcut_i = ff.sb[ti * SB_N + SB_BCUT_ACKS2], s_i = s_kin[i];
   const long long tag_i = d.tag[i];
   const int center = (d.S * d.S * d.S - 1) / 2;
   double gx = 0, gy = 0, gz = 0, ee = 0, eh2 = 0, v0 = 0, v1 = 0, v2 = 0, v3 = 0, v4 = 0, v5 = 0;
   for (int e = lane; e < cnt; e += 32) {
-    const unsigned code = d.nbr[static_cast<size_t>(i) * d.ncap + e];
-    const int j = static_cast<int>(code & d.amask);
+    const unsigned code = d.nbr[static_cast<size_t>(warp) * d.ncap + e];
+    const double4 xj = d.xr[code & d.amask];
+    const int j = ord_atom(xj);
     const int sidx = static_cast<int>(code >> d.abits);
-    const double xcut = 0.5 * (bcut_i + ff.sb[d.type[j] * SB_N + SB_BCUT_ACKS2]);
+    const double xcut = 0.5 * (bcut_i + ff.sb[ord_type(xj) * SB_N + SB_BCUT_ACKS2]);
     double dv[3];
-    pair_dvec(d, s, i, j, sidx, dv);
+    pair_dvec_x(d, s, i, j, sidx, xi4, xj, dv);
     const double dist = sqrt(dv[0] * dv[0] + dv[1] * dv[1] + dv[2] * dv[2]);
     if (!(dist <= xcut)) continue;
     const double dd = dist / xcut, om = 1.0 - dd, om2 = om * om;
@@ -663,150 +696,280 @@ __global__ void k_acks2(Dev d, DevFF ff, const double* s_kin) {
 }
 
 // ------------------------------------------------------------------------------------------------ QEq CG
-// y = (diag(eta) + H) v for one row, both right-hand sides (s, t) at once; warp per row, each lane taking four
-// consecutive entries per pass with 16-byte loads (rows start 128-byte aligned: ncap is a multiple of 32); H as
-// hi + lo (the FP64 matrix to ~1e-15).
-__device__ inline double2 row_mv(const Dev& d, int i, double eta, const double2* v) {
-  const int cnt = min(d.nbr_cnt[i], d.ncap);
+// The charge solve works in cell order throughout (vectors, rows, columns). Lanes take consecutive entries of a row, which
+// mostly name consecutive positions (the Verlet rows list runs of consecutive cells), so the 32 gathers of a load
+// touch a few cache lines instead of one each.
+//
+// (diag(eta) + H) v of one row in FP64 (hi + lo), in every lane
+__device__ inline double2 row_mv(const Dev& d, int p, double eta, const double2* v) {
   const int lane = threadIdx.x & 31;
-  const double2 vi = v[i];   // issued before the row so that its latency hides behind it
-  double ys = 0.0, yt = 0.0;
-  const size_t base = static_cast<size_t>(i) * d.ncap;
-  for (int e0 = lane * 4; e0 < cnt; e0 += 128) {
-    const uint4 c4 = *reinterpret_cast<const uint4*>(d.nbr + base + e0);
-    const float4 h4 = *reinterpret_cast<const float4*>(d.hhi + base + e0);
-    const float4 l4 = *reinterpret_cast<const float4*>(d.hlo + base + e0);
-    const unsigned cc[4] = {c4.x, c4.y, c4.z, c4.w};
-    const float hh[4] = {h4.x, h4.y, h4.z, h4.w}, ll[4] = {l4.x, l4.y, l4.z, l4.w};
+  const int cnt = d.nbr_cnt[p];
+  const double2 vi = v[p];   // issued before the row so that its latency hides behind it
+  const size_t base = static_cast<size_t>(p) * d.ncap;
+  double y[2] = {0.0, 0.0};
+  for (int e0 = lane; e0 < cnt; e0 += 128) {
+    unsigned c[4];
+    float hi[4], lo[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {   // past the row's end: weight 0 on the row's own vector entry
+      const int e = e0 + 32 * k;
+      const bool in = e < cnt;
+      c[k] = in ? d.nbr[base + e] & d.amask : static_cast<unsigned>(p);
+      hi[k] = in ? d.hhi[base + e] : 0.f;
+      lo[k] = in ? d.hlo[base + e] : 0.f;
+    }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      if (e0 + k < cnt) {
-        const double h = static_cast<double>(hh[k]) + static_cast<double>(ll[k]);
-        const double2 vj = v[cc[k] & d.amask];
-        ys += h * vj.x;
-        yt += h * vj.y;
-      }
+      const double h = static_cast<double>(hi[k]) + static_cast<double>(lo[k]);
+      const double2 vj = v[c[k]];
+      y[0] += h * vj.x;
+      y[1] += h * vj.y;
     }
   }
-  ys = warp_sum(ys);
-  yt = warp_sum(yt);
-  return make_double2(eta * vi.x + __shfl_sync(0xffffffffu, ys, 0), eta * vi.y + __shfl_sync(0xffffffffu, yt, 0));
+  const double t = warp_sums<2>(y);
+  return make_double2(eta * vi.x + __shfl_sync(0xffffffffu, t, 0), eta * vi.y + __shfl_sync(0xffffffffu, t, 16));
 }
 
-// (A v)_i of the single-precision-matrix iterations: FP32 values of the matrix (hhi) times the FP32 copy vf of v,
-// products and sums in FP64; the diagonal term takes v_i itself. Gathering 8-byte float2 halves the bytes of the
-// gathers (the vector of a 24k-atom system then fits in an SM's L1).
-__device__ inline double2 row_mv_f32(const Dev& d, int i, double eta, const double2* v, const float2* vf) {
-  const int cnt = min(d.nbr_cnt[i], d.ncap);
-  const int lane = threadIdx.x & 31;
-  const double2 vi = v[i];
-  double ys = 0.0, yt = 0.0;
-  const size_t base = static_cast<size_t>(i) * d.ncap;
-  for (int e0 = lane * 8; e0 < cnt; e0 += 256) {   // eight entries per lane in flight (rows hold ncap, a multiple of 32)
-    const uint4 c4a = *reinterpret_cast<const uint4*>(d.nbr + base + e0);
-    const uint4 c4b = *reinterpret_cast<const uint4*>(d.nbr + base + e0 + 4);
-    const float4 h4a = *reinterpret_cast<const float4*>(d.hhi + base + e0);
-    const float4 h4b = *reinterpret_cast<const float4*>(d.hhi + base + e0 + 4);
-    const unsigned cc[8] = {c4a.x, c4a.y, c4a.z, c4a.w, c4b.x, c4b.y, c4b.z, c4b.w};
-    const float hh[8] = {h4a.x, h4a.y, h4a.z, h4a.w, h4b.x, h4b.y, h4b.z, h4b.w};
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (e0 + k < cnt) {
-        const float2 vj = vf[cc[k] & d.amask];
-        ys += static_cast<double>(hh[k]) * static_cast<double>(vj.x);
-        yt += static_cast<double>(hh[k]) * static_cast<double>(vj.y);
-      }
-    }
-  }
-  ys = warp_sum(ys);
-  yt = warp_sum(yt);
-  return make_double2(eta * vi.x + __shfl_sync(0xffffffffu, ys, 0), eta * vi.y + __shfl_sync(0xffffffffu, yt, 0));
+// Row products of a warp's consecutive rows as one stream of 128-entry pieces. A row product alone is bound by latency:
+// the entries come from L2 or HBM (600-1000 cycles) and only then can the vector be gathered. Here the entries are
+// copied into a per-warp ring in shared memory several pieces ahead (cp.async: no registers, no waiting), and the gathers
+// of one piece run beside the copies of the next ones.
+static_assert(kRingBytes == 6 * 2 * 512 && kRingBytes == 4 * 3 * 512, "6 pieces of (column, hi), 4 of (column, hi, lo)");
+__device__ __forceinline__ void copy16_async(unsigned dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kLeft>
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory"); }
+
+// y[r] = sum over row p0 + r of H v (without the diagonal) for r < nrows, by one warp; cnt[r] entries in row p0 + r; V is
+// float2 (the FP32 copy of a vector, with the matrix's hi parts) or double2 (with hi + lo); products and sums FP64
+//
+// start() issues the first copies: before a grid barrier, so that the matrix is on its way while the blocks meet.
+template <bool kF64>
+struct RowStream {
+  static constexpr int kStages = kF64 ? 4 : 6, kStage = (kF64 ? 3 : 2) * 512;
+  const unsigned* col;
+  const float* hi;
+  const float* lo;
+  const int* cnt;
+  const char* ring;
+  int nrows, ncap;
+  int fr, fe, fn;       // the next piece to fetch: row, first entry, length of the row
+  unsigned fo, wr, ring_at;
+
+  __device__ __forceinline__ void next_row() {
+    fe = 0;
+    do {
+      ++fr;
+      fo += static_cast<unsigned>(ncap);
+      fn = fr < nrows ? cnt[fr] : 1;
+    } while (fn == 0);
+  }
+  __device__ __forceinline__ void fetch() {
+    const int lane = threadIdx.x & 31;
+    if (fr < nrows) {
+      if (fe + 4 * lane < fn) {   // rows hold a multiple of 32 entries: 16 bytes from a multiple of 4 stay inside
+        const unsigned o = fo + static_cast<unsigned>(fe);
+        copy16_async(wr, col + o);
+        copy16_async(wr + 512, hi + o);
+        if (kF64) copy16_async(wr + 1024, lo + o);
+      }
+      fe += 128;
+      if (fe >= fn) next_row();
+    }
+    copy_commit();   // an empty group past the end keeps the count of groups in step with the pieces
+    wr = wr + kStage == ring_at + kStages * kStage ? ring_at : wr + kStage;
+  }
+  // rows p0 .. p0 + rows - 1 of the matrix, cnt_[r] entries in row p0 + r
+  __device__ __forceinline__ void start(const Dev& d, int p0, int rows, const int* cnt_, const char* ring_) {
+    const int lane = threadIdx.x & 31;
+    const size_t base = static_cast<size_t>(p0) * d.ncap + 4 * lane;
+    col = d.nbr + base;
+    hi = d.hhi + base;
+    lo = d.hlo + base;
+    cnt = cnt_;
+    ring = ring_;
+    nrows = rows;
+    ncap = d.ncap;
+    ring_at = static_cast<unsigned>(__cvta_generic_to_shared(ring_)) + 16 * lane;
+    fr = 0;
+    fe = 0;
+    fo = 0;
+    wr = ring_at;
+    fn = nrows > 0 ? cnt[0] : 0;
+    if (nrows > 0 && fn == 0) next_row();
+#pragma unroll
+    for (int s = 0; s < kStages - 1; ++s) fetch();
+  }
+  // y[r] = sum over row p0 + r of H v (without the diagonal); V is float2 (the FP32 copy of a vector, with the matrix's hi
+  // parts) or double2 (with hi + lo); products and sums FP64
+  template <class V>
+  __device__ __forceinline__ void run(unsigned amask, int p0, const V* v, double2* y) {
+    const int lane = threadIdx.x & 31;
+    unsigned rd = 0;
+    for (int r = 0; r < nrows; ++r) {
+      const int n = cnt[r];
+      double acc[2] = {0.0, 0.0};
+      auto piece = [&](int left, auto whole) {   // `left` entries of the row from here on; whole: 128 or more
+        copy_wait<kStages - 2>();
+        __syncwarp();
+        const char* at = ring + rd + 4 * lane;
+        unsigned c[4];
+        float h[4], l[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          c[k] = *reinterpret_cast<const unsigned*>(at + 128 * k) & amask;
+          h[k] = *reinterpret_cast<const float*>(at + 512 + 128 * k);
+          if (kF64) l[k] = *reinterpret_cast<const float*>(at + 1024 + 128 * k);
+          if (!decltype(whole)::value && lane + 32 * k >= left) {   // past the end: weight 0 on the row's own vector entry
+            c[k] = static_cast<unsigned>(p0 + r);
+            h[k] = 0.f;
+            if (kF64) l[k] = 0.f;
+          }
+        }
+        V w[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) w[k] = v[c[k]];
+        fetch();   // into the piece read before this one (every lane has passed the barrier above since)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const double m = kF64 ? static_cast<double>(h[k]) + static_cast<double>(l[k]) : static_cast<double>(h[k]);
+          acc[0] += m * static_cast<double>(w[k].x);
+          acc[1] += m * static_cast<double>(w[k].y);
+        }
+        rd = rd + kStage == kStages * kStage ? 0u : rd + kStage;
+      };
+      int e = 0;
+      for (; e + 128 <= n; e += 128) piece(128, std::true_type{});
+      if (e < n) piece(n - e, std::false_type{});
+      const double s = warp_sums<2>(acc);
+      if ((lane & 15) == 0) reinterpret_cast<double*>(y + r)[lane >> 4] = s;
+    }
+    copy_wait<0>();
+    __syncwarp();
+  }
+};
 
 // deterministic block sum of NV doubles per thread into out[blockIdx.x * NV + k]
 template <int NV>
-__device__ inline void block_partials(const double* v, double* out, double* sh) {
+__device__ inline void block_partials(double* v, double* out, double* sh) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int k = 0; k < NV; ++k) {
-    double x = v[k];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[wid * NV + k] = x;
-  }
+  const double t = warp_sums<NV>(v);
+  if ((lane & (32 / NV - 1)) == 0) sh[wid * NV + lane / (32 / NV)] = t;
   __syncthreads();
-  if (threadIdx.x < NV) {
-    double t = 0.0;
-    for (int w = 0; w < nw; ++w) t += sh[w * NV + threadIdx.x];
-    out[blockIdx.x * NV + threadIdx.x] = t;
+  if (wid == 0) {
+    double u[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) u[k] = lane < nw ? sh[lane * NV + k] : 0.0;
+    const double s = warp_sums<NV>(u);
+    if ((lane & (32 / NV - 1)) == 0) out[blockIdx.x * NV + lane / (32 / NV)] = s;
   }
-  __syncthreads();
 }
 
-// Sum of the per-block partials, identical in every block: each thread loads a strided subset in order, then a
-// fixed-shape shuffle tree and a fixed-order sum over the warps (the tree depends only on gridDim and blockDim).
+// Sum of the per-block partials, the same in every block: each lane of the first warp sums a strided subset in order, then a
+// fixed exchange (the order depends only on the number of blocks). Read around L1: another block wrote them. One warp
+// per block reads them (the partials are a few cache lines: read by every warp of the grid they take 5 us more).
 template <int NV>
 __device__ inline void grid_totals(const double* part, int nblocks, double* tot, double* sh) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int k = 0; k < NV; ++k) {
-    double t = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) t += part[b * NV + k];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-    if (lane == 0) sh[wid * NV + k] = t;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) {
+    double v[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = 0.0;
+    for (int b = lane; b < nblocks; b += 32) {
+#pragma unroll
+      for (int k = 0; k < NV; k += 2) {
+        const double2 t = __ldcg(reinterpret_cast<const double2*>(part + b * NV + k));
+        v[k] += t.x;
+        v[k + 1] += t.y;
+      }
+    }
+    const double t = warp_sums<NV>(v);
+    if ((lane & (32 / NV - 1)) == 0) sh[lane / (32 / NV)] = t;
   }
   __syncthreads();
-  for (int k = 0; k < NV; ++k) {
-    double t = 0.0;
-    for (int w = 0; w < nw; ++w) t += sh[w * NV + k];
-    tot[k] = t;
-  }
-  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) tot[k] = sh[k];
 }
 
-// Persistent cooperative Jacobi-PCG for one system, s and t solved together: the stock loop of fix qeq/reaxff as
-// reproduced in plugin/adapter/fix_qeq_reaxff_metal.cpp:89-123, each right-hand side stopping on its own test
+// Persistent cooperative Jacobi-PCG for one system, s and t solved together: the loop of fix qeq/reaxff as reproduced in
+// plugin/adapter/fix_qeq_reaxff_metal.cpp:89-123, each right-hand side stopping on its own test
 // sqrt(r.M^-1 r)/|b| <= tol with at most imax-1 iterations; then calculate_Q: q = s - (sum s / sum t) t.
 // Precision (the resident refinement of src/metal/metal_backend.mm:435-530, in FP64 instead of double-single): the
-// iterations multiply the single-precision matrix (hi: 8 bytes per entry with its index) by an FP32 copy of the search
-// direction (products and sums in FP64), the vectors and every dot product are FP64, and the residual is recomputed with the FP64 matrix (hi + lo) whenever the iterations have
-// converged - or have reduced the residual by kRefineDrop, below which the single-precision matrix stops helping. The
-// solve ends only on that FP64 residual, so the tolerance and the reported residuals are those of the FP64 system.
-// Rows are distributed over all warps of the grid; reductions are fixed-order (per-block partials summed in block
-// order), so the result is bitwise reproducible. Only grid.sync() waits; the kernel is launched cooperatively.
+// iterations multiply the single-precision matrix (hi: 8 bytes per entry with its index) by an FP32 copy of the
+// preconditioned residual (products and sums in FP64), the vectors and every dot product are FP64, and the residual is
+// recomputed with the FP64 matrix (hi + lo) whenever the iterations have converged - or have reduced the residual by
+// kRefineDrop, below which the single-precision matrix stops helping. The solve ends only on that FP64 residual, so the
+// tolerance and the reported residuals are those of the FP64 system.
+//
+// Every block owns a contiguous range of cell-ordered rows and keeps their vectors in shared memory; other blocks read
+// only the copy `df` of u = M^-1 r. The iteration is the form of Chronopoulos and Gear (J. Comput. Appl. Math. 25, 153
+// (1989)): w = A u, then d = u + beta d and A d = w + beta (A d) by recurrence, so that only two grid barriers are
+// needed per iteration (after the row products, carrying u.w, and after the vector update, carrying the new r.u)
+// instead of three. Reductions are fixed-order, so the result is bitwise reproducible. Only grid.sync() waits; the
+// kernel is launched cooperatively.
 constexpr double kRefineDrop = 1e-6;
 
 __global__ void __launch_bounds__(1024, 1) k_cg_grid(Dev d, CgArgs a) {
   cg::grid_group g = cg::this_grid();
+  // a ring per warp; then, when they fit, the six vectors and the row lengths of the block's rows (else in global memory)
+  extern __shared__ double2 dyn[];
   __shared__ double sh[32 * 4];
-  __shared__ double tot_sh[32 * 4];
-  const int wpb = blockDim.x >> 5;
-  const int gw = blockIdx.x * wpb + (threadIdx.x >> 5);
-  const int nwarps = gridDim.x * wpb;
-  const int lane = threadIdx.x & 31;
-  const int i0 = a.begin, n = a.n;
+  __shared__ double tot_sh[4];
+  const int n = a.n, nb = static_cast<int>(gridDim.x), blk = static_cast<int>(blockIdx.x);
+  const int r0 = static_cast<int>(static_cast<long long>(n) * blk / nb), r1 = static_cast<int>(static_cast<long long>(n) * (blk + 1) / nb);
+  const int m = r1 - r0;
+  const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int w0 = m * wid / nw, w1 = m * (wid + 1) / nw;   // this warp's rows (within the block's)
+  char* ring = reinterpret_cast<char*>(dyn) + wid * kRingBytes;
+  double2* vec = dyn + nw * (kRingBytes / sizeof(double2));
+  double* etas = reinterpret_cast<double*>(vec + 6 * static_cast<size_t>(a.smem_rows));
+  int* cnts = reinterpret_cast<int*>(etas + a.smem_rows);
+  const double* E = a.smem_rows ? etas : a.eta + r0;
+  const int* cnt = a.smem_rows ? cnts : d.nbr_cnt + r0;
+  double2* X = a.smem_rows ? vec : a.x + r0;
+  double2* R = a.smem_rows ? vec + a.smem_rows : a.r + r0;
+  double2* U = a.smem_rows ? vec + 2 * a.smem_rows : a.p + r0;
+  double2* W = a.smem_rows ? vec + 3 * a.smem_rows : a.q + r0;
+  double2* D = a.smem_rows ? vec + 4 * a.smem_rows : a.d + r0;
+  double2* S = a.smem_rows ? vec + 5 * a.smem_rows : a.s + r0;
   double loc[4], tot[4];
   int phase = 0;
-  auto partbuf = [&]() { return a.part + static_cast<size_t>(phase & 1) * gridDim.x * 4; };
+  auto partbuf = [&]() { return a.part + static_cast<size_t>(phase & 1) * nb * 4; };
   double bnorm_s = 0.0, bnorm_t = 0.0, sig_s = 0.0, sig_t = 0.0;
   bool act_s = true, act_t = true, breakdown = false;
   int it_s = 1, it_t = 1, nref = 0;
+  for (int k = threadIdx.x; k < m; k += blockDim.x) {
+    X[k] = a.x[r0 + k];
+    if (a.smem_rows) {
+      etas[k] = a.eta[r0 + k];
+      cnts[k] = d.nbr_cnt[r0 + k];
+    }
+  }
+  __syncthreads();
+  RowStream<true> exact;
+  RowStream<false> fast;
+  exact.start(d, r0 + w0, w1 - w0, cnt + w0, ring);
   for (;;) {
-    // ---- FP64 residual: r = b - A x ; p = M^-1 r ; r.p (and |b|^2 on the first pass)
+    // ---- FP64 residual: r = b - A x ; u = M^-1 r ; r.u (and |b|^2 on the first pass)
+    exact.run(d.amask, r0 + w0, a.x, W + w0);
+    __syncthreads();
     loc[0] = loc[1] = loc[2] = loc[3] = 0.0;
-    for (int r = gw; r < n; r += nwarps) {
-      const int i = i0 + r;
-      const double eta = a.eta[i];
-      const double2 y = row_mv(d, i, eta, a.x);
-      if (lane == 0) {
-        const double2 b = a.b[i];
-        const double2 rr = make_double2(b.x - y.x, b.y - y.y);
-        a.r[i] = rr;
-        const double2 pp = make_double2(rr.x / eta, rr.y / eta);
-        a.p[i] = pp;
-        loc[0] += b.x * b.x; loc[1] += b.y * b.y; loc[2] += rr.x * pp.x; loc[3] += rr.y * pp.y;
-      }
+    for (int k = threadIdx.x; k < m; k += blockDim.x) {
+      const double eta = E[k];
+      const double2 b = a.b[r0 + k], x = X[k], y = W[k];
+      const double2 r = make_double2(b.x - (eta * x.x + y.x), b.y - (eta * x.y + y.y));
+      const double2 u = make_double2(r.x / eta, r.y / eta);
+      R[k] = r;
+      U[k] = u;
+      a.df[r0 + k] = make_float2(static_cast<float>(u.x), static_cast<float>(u.y));
+      loc[0] += b.x * b.x; loc[1] += b.y * b.y; loc[2] += r.x * u.x; loc[3] += r.y * u.y;
     }
     block_partials<4>(loc, partbuf(), sh);
+    fast.start(d, r0 + w0, w1 - w0, cnt + w0, ring);
     g.sync();
-    grid_totals<4>(partbuf(), gridDim.x, tot, tot_sh);
+    grid_totals<4>(partbuf(), nb, tot, tot_sh);
     ++phase;
     ++nref;
     if (nref == 1) { bnorm_s = sqrt(tot[0]); bnorm_t = sqrt(tot[1]); }
@@ -817,89 +980,90 @@ __global__ void __launch_bounds__(1024, 1) k_cg_grid(Dev d, CgArgs a) {
     if ((!act_s || it_s >= a.imax) && (!act_t || it_t >= a.imax)) break;
     const double stop_s = fmax(a.tol * bnorm_s, kRefineDrop * sqrt(sig_s));
     const double stop_t = fmax(a.tol * bnorm_t, kRefineDrop * sqrt(sig_t));
-    // ---- single-precision-matrix iterations from this residual (d = p on entry)
-    for (int r = gw * 32 + lane; r < n; r += nwarps * 32) {
-      const double2 pp = a.p[i0 + r];
-      a.d[i0 + r] = pp;
-      a.df[i0 + r] = make_float2(static_cast<float>(pp.x), static_cast<float>(pp.y));
-    }
-    g.sync();
-    for (;;) {
+    // ---- single-precision-matrix iterations from this residual
+    double beta_s = 0.0, beta_t = 0.0, alpha_s = 0.0, alpha_t = 0.0;
+    for (bool fresh = true;; fresh = false) {
       const bool in_s = act_s && it_s < a.imax && sqrt(sig_s) > stop_s;
       const bool in_t = act_t && it_t < a.imax && sqrt(sig_t) > stop_t;
       if (!in_s && !in_t) break;
-      // q = A d ; partial d.q
+      // w = A u ; partial u.w
+      fast.run(d.amask, r0 + w0, a.df, W + w0);
+      __syncthreads();
       loc[0] = loc[1] = 0.0;
-      for (int r = gw; r < n; r += nwarps) {
-        const int i = i0 + r;
-        const double2 y = row_mv_f32(d, i, a.eta[i], a.d, a.df);
-        if (lane == 0) {
-          a.q[i] = y;
-          const double2 dd = a.d[i];
-          loc[0] += dd.x * y.x; loc[1] += dd.y * y.y;
-        }
+      for (int k = threadIdx.x; k < m; k += blockDim.x) {
+        const double eta = E[k];
+        const double2 u = U[k];
+        double2 w = W[k];
+        w.x += eta * u.x; w.y += eta * u.y;
+        W[k] = w;
+        loc[0] += u.x * w.x; loc[1] += u.y * w.y;
       }
       block_partials<2>(loc, partbuf(), sh);
       g.sync();
-      grid_totals<2>(partbuf(), gridDim.x, tot, tot_sh);
+      grid_totals<2>(partbuf(), nb, tot, tot_sh);
       ++phase;
-      const double alpha_s = in_s ? sig_s / tot[0] : 0.0;
-      const double alpha_t = in_t ? sig_t / tot[1] : 0.0;
+      // d.Ad = u.w - beta r.u / (the previous step length); beta is 0 on the first iteration from a residual
+      const double bs = in_s ? beta_s : 0.0, bt = in_t ? beta_t : 0.0;
+      alpha_s = in_s ? sig_s / (fresh ? tot[0] : tot[0] - bs * sig_s / alpha_s) : 0.0;
+      alpha_t = in_t ? sig_t / (fresh ? tot[1] : tot[1] - bt * sig_t / alpha_t) : 0.0;
       if (!(isfinite(alpha_s) && isfinite(alpha_t))) { breakdown = true; break; }
-      // x += alpha d ; r -= alpha q ; p = M^-1 r ; partial r.p
+      // d = u + beta d ; Ad = w + beta Ad ; x += alpha d ; r -= alpha Ad ; u = M^-1 r ; partial r.u
       loc[0] = loc[1] = 0.0;
-      for (int r = gw * 32 + lane; r < n; r += nwarps * 32) {
-        const int i = i0 + r;
-        const double2 dd = a.d[i], qq = a.q[i];
-        double2 xx = a.x[i], rr = a.r[i];
-        xx.x += alpha_s * dd.x; xx.y += alpha_t * dd.y;
-        rr.x -= alpha_s * qq.x; rr.y -= alpha_t * qq.y;
-        a.x[i] = xx;
-        a.r[i] = rr;
-        const double eta = a.eta[i];
-        const double2 pp = make_double2(rr.x / eta, rr.y / eta);
-        a.p[i] = pp;
-        loc[0] += rr.x * pp.x; loc[1] += rr.y * pp.y;
+      for (int k = threadIdx.x; k < m; k += blockDim.x) {
+        const double eta = E[k];
+        const double2 w = W[k];
+        double2 u = U[k], dd = u, ss = w, x = X[k], r = R[k];
+        if (!fresh) {   // a right-hand side that has stopped keeps beta = 0: its vectors stay finite, its step is 0
+          const double2 o = D[k], q = S[k];
+          dd.x += bs * o.x; dd.y += bt * o.y;
+          ss.x += bs * q.x; ss.y += bt * q.y;
+        }
+        D[k] = dd;
+        S[k] = ss;
+        x.x += alpha_s * dd.x; x.y += alpha_t * dd.y;
+        r.x -= alpha_s * ss.x; r.y -= alpha_t * ss.y;
+        u = make_double2(r.x / eta, r.y / eta);
+        X[k] = x;
+        R[k] = r;
+        U[k] = u;
+        a.df[r0 + k] = make_float2(static_cast<float>(u.x), static_cast<float>(u.y));
+        loc[0] += r.x * u.x; loc[1] += r.y * u.y;
       }
       block_partials<2>(loc, partbuf(), sh);
+      fast.start(d, r0 + w0, w1 - w0, cnt + w0, ring);
       g.sync();
-      grid_totals<2>(partbuf(), gridDim.x, tot, tot_sh);
+      grid_totals<2>(partbuf(), nb, tot, tot_sh);
       ++phase;
-      const double beta_s = in_s ? tot[0] / sig_s : 0.0;
-      const double beta_t = in_t ? tot[1] / sig_t : 0.0;
-      if (in_s) { sig_s = tot[0]; ++it_s; }
-      if (in_t) { sig_t = tot[1]; ++it_t; }
-      // d = p + beta d (only for the right-hand sides still iterating)
-      for (int r = gw * 32 + lane; r < n; r += nwarps * 32) {
-        const int i = i0 + r;
-        const double2 pp = a.p[i];
-        double2 dd = a.d[i];
-        if (in_s) dd.x = pp.x + beta_s * dd.x;
-        if (in_t) dd.y = pp.y + beta_t * dd.y;
-        a.d[i] = dd;
-        a.df[i] = make_float2(static_cast<float>(dd.x), static_cast<float>(dd.y));
-      }
-      g.sync();
+      if (in_s) { beta_s = tot[0] / sig_s; sig_s = tot[0]; ++it_s; }
+      if (in_t) { beta_t = tot[1] / sig_t; sig_t = tot[1]; ++it_t; }
     }
+    for (int k = threadIdx.x; k < m; k += blockDim.x) a.x[r0 + k] = X[k];
     if (breakdown) break;
+    copy_wait<0>();   // the pieces of the pass that is not taken, before the ring is filled anew
+    __syncwarp();
+    exact.start(d, r0 + w0, w1 - w0, cnt + w0, ring);
+    g.sync();   // the FP64 residual reads every block's solution
   }
+  copy_wait<0>();
   // calculate_Q: q = s - (sum s / sum t) t
   loc[0] = loc[1] = 0.0;
-  for (int r = gw * 32 + lane; r < n; r += nwarps * 32) {
-    const double2 xx = a.x[i0 + r];
-    loc[0] += xx.x; loc[1] += xx.y;
+  for (int k = threadIdx.x; k < m; k += blockDim.x) {
+    const double2 x = X[k];
+    loc[0] += x.x; loc[1] += x.y;
   }
   block_partials<2>(loc, partbuf(), sh);
   g.sync();
-  grid_totals<2>(partbuf(), gridDim.x, tot, tot_sh);
+  grid_totals<2>(partbuf(), nb, tot, tot_sh);
   ++phase;
   const double u = tot[0] / tot[1];
   if (a.write_q)
-    for (int r = gw * 32 + lane; r < n; r += nwarps * 32) {
-      const double2 xx = a.x[i0 + r];
-      d.q[i0 + r] = xx.x - u * xx.y;
+    for (int k = threadIdx.x; k < m; k += blockDim.x) {
+      const double2 x = X[k];
+      const double q = x.x - u * x.y;
+      d.qr[r0 + k] = q;
+      d.q[d.cell_atoms[r0 + k]] = q;
     }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (blk == 0 && threadIdx.x == 0) {
     if (a.out_brk) a.out_brk[0] = breakdown ? 1 : 0;
     a.out_iters[0] = it_s;
     a.out_iters[1] = it_t;
@@ -1122,7 +1286,9 @@ __global__ void __launch_bounds__(256, 4) k_cg_seg(Dev d, CgArgs a) {
     if (a.write_q)
       for (int k = lane; k < si.natoms; k += 32) {
         const double2 xx = a.x[si.begin + k];
-        d.q[si.begin + k] = xx.x - u * xx.y;
+        const double qq = xx.x - u * xx.y;
+        d.qr[si.begin + k] = qq;
+        d.q[d.cell_atoms[si.begin + k]] = qq;
       }
     if (lane == 0) {
       const SysCg& c = a.sc[s];
@@ -1141,11 +1307,11 @@ __global__ void __launch_bounds__(256, 4) k_cg_seg(Dev d, CgArgs a) {
 // Initial guesses from the histories (Q-23: s = 4(s0+s2) - (6 s1 + s3), t = t2 + 3(t0 - t1); index 0 = latest),
 // right-hand sides b_s = -chi, b_t = -1, and the diagonal eta.
 __global__ void k_qeq_prepare(Dev d, DevFF ff, CgArgs a, const double* s_hist, const double* t_hist) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;   // cell-order position
   if (i >= d.na) return;
-  const int t = d.type[i];
-  const double* sh = s_hist + 4 * static_cast<size_t>(i);
-  const double* th = t_hist + 4 * static_cast<size_t>(i);
+  const int atom = d.cell_atoms[i], t = d.type[atom];
+  const double* sh = s_hist + 4 * static_cast<size_t>(atom);
+  const double* th = t_hist + 4 * static_cast<size_t>(atom);
   a.x[i] = make_double2(4 * (sh[0] + sh[2]) - (6 * sh[1] + sh[3]), th[2] + 3 * (th[0] - th[1]));
   a.b[i] = make_double2(-ff.sb[t * SB_N + SB_CHI], -1.0);
   a.eta[i] = ff.sb[t * SB_N + SB_ETA];
@@ -1156,9 +1322,10 @@ __global__ void k_qeq_prepare(Dev d, DevFF ff, CgArgs a, const double* s_hist, c
 __global__ void k_qeq_prepare_given(Dev d, DevFF ff, CgArgs a, const double* b, const double* x0) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.na) return;
-  a.x[i] = x0 ? make_double2(x0[i], x0[d.na + i]) : make_double2(0.0, 0.0);
-  a.b[i] = make_double2(b[i], b[d.na + i]);
-  a.eta[i] = ff.sb[d.type[i] * SB_N + SB_ETA];
+  const int atom = d.cell_atoms[i];
+  a.x[i] = x0 ? make_double2(x0[atom], x0[d.na + atom]) : make_double2(0.0, 0.0);
+  a.b[i] = make_double2(b[atom], b[d.na + atom]);
+  a.eta[i] = ff.sb[d.type[atom] * SB_N + SB_ETA];
 }
 
 // the solve just finished becomes the newest history entry; not after a list overflow (the evaluation is repeated),
@@ -1173,17 +1340,28 @@ __global__ void k_qeq_history(Dev d, const double2* x, double* s_hist, double* t
   double* sh = s_hist + 4 * static_cast<size_t>(i);
   double* th = t_hist + 4 * static_cast<size_t>(i);
   for (int k = 3; k > 0; --k) { sh[k] = sh[k - 1]; th[k] = th[k - 1]; }
-  sh[0] = x[i].x;
-  th[0] = x[i].y;
+  const double2 xi = x[d.rank[i]];
+  sh[0] = xi.x;
+  th[0] = xi.y;
 }
 
-// y = (diag(eta) + H) v, owned rows (mtl::Context::qeq_matvec)
+// y = (diag(eta) + H) v, owned rows (mtl::Context::qeq_matvec): v in cell order, y by atom
 __global__ void k_qeq_matvec(Dev d, DevFF ff, const double2* v, double2* y) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (warp >= d.na) return;
-  const double eta = ff.sb[d.type[warp] * SB_N + SB_ETA];
+  const double eta = ff.sb[ord_type(d.xr[warp]) * SB_N + SB_ETA];
   const double2 r = row_mv(d, warp, eta, v);
-  if ((threadIdx.x & 31) == 0) y[warp] = r;
+  if ((threadIdx.x & 31) == 0) y[ord_atom(d.xr[warp])] = r;
+}
+
+// per-atom values into cell order and back
+__global__ void k_to_cell_order(Dev d, const double2* by_atom, double2* by_position) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < d.na) by_position[p] = by_atom[d.cell_atoms[p]];
+}
+__global__ void k_to_atom_order(Dev d, const double2* by_position, double2* by_atom) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < d.na) by_atom[d.cell_atoms[p]] = by_position[p];
 }
 
 // ------------------------------------------------------------------------------------------------ energy sums
