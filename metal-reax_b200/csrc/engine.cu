@@ -159,6 +159,9 @@ struct Context {
   DBuf<double> cg_eta, cg_part, s_hist, t_hist, cg_rel;
   DBuf<int> cg_iters, cg_nlive, cg_nref, cg_brk;
   DBuf<SysCg> cg_sys;
+  DBuf<int> cg_order, cg_ticket;   // systems of up to kClusterAtoms atoms, largest first; the clusters' counter
+  int n_small = 0, max_small = 0;
+  long long rows_small = 0;
   DBuf<double2> cg_rb0, cg_rb1;
   std::vector<int> last_iters;
   std::vector<double> last_rel;
@@ -636,6 +639,23 @@ struct Context {
     fown_h.ensure(n); fown_t.ensure(n); fix_h.ensure(3 * n); pe_fix.ensure(n);
     cg_x.ensure(n); cg_df.ensure(n); cg_b.ensure(n); cg_r.ensure(n); cg_d.ensure(n); cg_p.ensure(n); cg_q.ensure(n); cg_s.ensure(n); cg_eta.ensure(n);
     cg_iters.ensure(2 * static_cast<size_t>(nsys)); cg_rel.ensure(2 * static_cast<size_t>(nsys));
+    {
+      std::vector<int> order;
+      rows_small = 0;
+      max_small = 0;
+      for (int s = 0; s < nsys; ++s) {
+        const int k = hsys[static_cast<size_t>(s)].natoms;
+        if (k > kClusterAtoms) continue;
+        order.push_back(s);
+        rows_small += k;
+        max_small = std::max(max_small, k);
+      }
+      n_small = static_cast<int>(order.size());
+      std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return hsys[static_cast<size_t>(x)].natoms > hsys[static_cast<size_t>(y)].natoms; });
+      cg_order.ensure(order.size());
+      cg_ticket.ensure(1);
+      if (n_small > 0) RXCU(cudaMemcpy(cg_order.p, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice));
+    }
     cg_sys.ensure(nsys); cg_rb0.ensure(n); cg_rb1.ensure(n); cg_nlive.ensure(2);
     cg_part.ensure(16 * static_cast<size_t>(std::max(nsm, 1)) * 32);
   }
@@ -804,6 +824,63 @@ struct Context {
   } tune;
   int grid_occ[5] = {0, 0, 0, 0, 0}, seg_per_sm = 0;
   static constexpr int kCgSmem = 220 * 1024;   // dynamic shared memory of the single-system CG at most
+
+  // ---- the cluster solve's launch shape (no result bit depends on it)
+  static constexpr int kClusterThreads = 512;
+  int cluster_fit[17] = {};   // clusters of that many blocks that the GPU holds at once (-1: none), once asked for
+  static int cluster_rows(int natoms, int c) {   // the most rows a block of the cluster owns: whole groups of eight
+    const int groups = (natoms + 7) / 8;
+    return 8 * ((groups + c - 1) / c);
+  }
+  static size_t cluster_smem(int natoms, int c) {
+    return static_cast<size_t>(kClusterThreads / 32) * kRingBytes + 3 * (kClusterAtoms / 8) * sizeof(double2) + 92 * static_cast<size_t>(cluster_rows(natoms, c));
+  }
+  cudaLaunchConfig_t cluster_config(int c, cudaLaunchAttribute* at) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(c));
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = cluster_smem(max_small, c);
+    cfg.stream = stream;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = static_cast<unsigned>(c);
+    at->val.clusterDim.y = 1;
+    at->val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+  }
+  // The cluster size with the shortest expected solve. An iteration of a system of n rows on c blocks takes about
+  // kRowUs n / c + kMeetUs; the clusters share the systems, and none ends before the largest system's. Measured, us a
+  // solve on 2, 4, 8, 16 blocks: 512 CHO systems of 64-1024 atoms 6925, 7235, 10885, 17918; 16 of 100-5000 (those up to
+  // 4096) 8: 2893, 16: 1542; one of 648 atoms 422, 250, 164, 116.
+  int cluster_size() {
+    constexpr double kRowUs = 0.25, kMeetUs = 4.0;
+    int best = 0;
+    double least = 0.0;
+    for (int c : {16, 8, 4, 2}) {
+      if (cluster_smem(max_small, c) > static_cast<size_t>(kCgSmem)) continue;
+      if (!cluster_fit[c]) {
+        RXCU(cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgSmem));
+        RXCU(cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchAttribute at;
+        cudaLaunchConfig_t cfg = cluster_config(c, &at);
+        cfg.dynamicSmemBytes = kCgSmem;
+        int fits = 0;
+        if (cudaOccupancyMaxActiveClusters(&fits, k_cg_cluster, &cfg) != cudaSuccess) {
+          (void)cudaGetLastError();
+          fits = 0;
+        }
+        cluster_fit[c] = fits > 0 ? fits : -1;
+      }
+      if (cluster_fit[c] < 0) continue;
+      const int g = std::min(n_small, cluster_fit[c]);
+      const double t = std::max((kRowUs * rows_small / c + kMeetUs * n_small) / g, kRowUs * max_small / c + kMeetUs);
+      if (!best || t < least) { best = c; least = t; }
+    }
+    if (!best) throw Error(RX_ERR_CUDA, "no thread-block cluster of the charge solve fits the GPU");
+    return best;
+  }
+
   void launch_cg(const Dev& d, CgArgs a) {
     if (nsys == 1 && na > tune.lone_grid_min) {   // one large system: all SMs on its rows, block partials in block order
       const int units = tune.cg_per_sm > 0 ? std::min(tune.cg_per_sm, 4) : 4;
@@ -824,7 +901,20 @@ struct Context {
       void* args[] = {const_cast<Dev*>(&d), &a};
       ++launches;
       RXCU(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_cg_grid), dim3(grid), dim3(threads), args, smem, stream));
-    } else {   // a batch (or one small system): every row of every system on all SMs, per-system fixed-order sums
+      return;
+    }
+    if (n_small > 0) {   // every system of up to kClusterAtoms atoms, alone or in a batch, by a cluster
+      const int c = cluster_size();
+      a.order = cg_order.p; a.nsmall = n_small; a.ticket = cg_ticket.p;
+      a.smem_rows = cluster_rows(max_small, c);
+      cudaLaunchAttribute at;
+      cudaLaunchConfig_t cfg = cluster_config(c, &at);
+      cfg.gridDim = dim3(static_cast<unsigned>(c * std::min(n_small, std::max(1, cluster_fit[c]))));
+      RXCU(cudaMemsetAsync(cg_ticket.p, 0, sizeof(int), stream));
+      ++launches;
+      RXCU(cudaLaunchKernelEx(&cfg, k_cg_cluster, d, a));
+    }
+    if (n_small < nsys) {   // the larger systems of a batch: every row of every one on all SMs, per-system fixed-order sums
       const int threads = 256;
       if (!seg_per_sm) RXCU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&seg_per_sm, k_cg_seg, threads, 0));
       int grid = std::max(1, std::min(seg_per_sm * nsm, (na + (threads / 32) - 1) / (threads / 32)));

@@ -20,6 +20,7 @@ struct SysCg {
   unsigned counter;   // rows of this system that have arrived in the current pass
 };
 
+constexpr int kClusterAtoms = 4096;   // systems of up to this many atoms are solved by a thread-block cluster each
 constexpr int kRingBytes = 6144;   // shared memory per warp of the charge solve's row products (rows_stream)
 
 struct CgArgs {
@@ -33,7 +34,7 @@ struct CgArgs {
   double2* q;
   double2* s;      // A d (single-system CG)
   float2* df;      // FP32 copy of M^-1 r, gathered by the single-precision-matrix iterations (single-system CG)
-  int smem_rows;   // rows per block whose vectors fit its shared memory (single-system CG; 0: vectors in global memory)
+  int smem_rows;   // rows per block whose vectors its shared memory holds (single-system CG; 0: vectors in global memory)
   double* eta;
   double* part;    // 2 * 8 * gridDim.x partial sums (double-buffered)
   int* out_iters;
@@ -41,6 +42,10 @@ struct CgArgs {
   int* out_nref;   // FP64 residual passes of the last single-system solve (may be null)
   int* out_brk;    // per system: 1 after a breakdown (a step length that is not finite)
   int write_q;     // 1: calculate_Q into the charges (the fix's solve); 0: solutions only
+  // cluster CG only: the systems it solves, largest first, their number, and the counter the clusters take them by
+  const int* order;
+  int nsmall;
+  int* ticket;
   // segmented CG only
   SysCg* sc;       // nsys
   double2* rb0;    // per-row dot-product terms (fixed-order per-system sums)
@@ -59,6 +64,7 @@ __global__ void k_nonbonded_half(Dev d, DevFF ff);
 __global__ void k_count_pairs(Dev d);
 __global__ void k_acks2(Dev d, DevFF ff, const double* s_kin);
 __global__ void k_cg_grid(Dev d, CgArgs a);
+__global__ void k_cg_cluster(Dev d, CgArgs a);
 __global__ void k_cg_seg(Dev d, CgArgs a);
 __global__ void k_qeq_prepare(Dev d, DevFF ff, CgArgs a, const double* s_hist, const double* t_hist);
 __global__ void k_qeq_prepare_given(Dev d, DevFF ff, CgArgs a, const double* b, const double* x0);

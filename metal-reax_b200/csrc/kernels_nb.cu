@@ -293,7 +293,10 @@ __global__ void __launch_bounds__(256) k_pairs(Dev d, DevFF ff, QeqParams qp) {
   const int warp = gid >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= d.na) return;
-  if (lists_failed(d)) return;
+  if (lists_failed(d)) {   // the evaluation is repeated: empty rows keep the kernels after this one inside the lists
+    if (lane == 0) d.nbr_cnt[warp] = 0;
+    return;
+  }
   const SysInfo s = d.sys[d.sys_of[warp]];
   const double rc2 = ff.nonb_cut * ff.nonb_cut;
   const double4 xi = d.xr[warp];
@@ -1075,7 +1078,188 @@ __global__ void __launch_bounds__(1024, 1) k_cg_grid(Dev d, CgArgs a) {
   }
 }
 
-// Segmented Jacobi-PCG: every system of the batch at once on one cooperative grid, the same algorithm (and the same
+// Jacobi-PCG of the systems of up to kClusterAtoms atoms, one thread-block cluster per system at a time (the clusters take
+// systems off a list, the largest first): the loop and the stopping rule of fix qeq/reaxff
+// (fix_qeq_reaxff_metal.cpp:89-123), s and t together, FP64 throughout (matrix hi + lo, vectors, dot products). The loop
+// keeps its three meetings an iteration: the two-barrier form of k_cg_grid gained 6 us of 122 at 648 atoms and nothing
+// on a batch. A solve over all SMs, however small the system, costs a grid barrier (5 us) or two
+// for every matrix pass of a microsecond or so, and a batch iterates until its last system has converged; a cluster's
+// hardware barrier costs about 1 us and each system stops on its own.
+//
+// A system's bits do not depend on the size of the cluster or on what else is in the batch: a row product depends on
+// the row alone, and every dot product is summed over groups of eight consecutive rows (a fixed exchange), the groups'
+// sums being handed to every block of the cluster and added up in one fixed order.
+constexpr int kGroup = 8;   // rows whose terms are summed before they are handed over
+__global__ void __launch_bounds__(512, 2) k_cg_cluster(Dev d, CgArgs a) {
+  cg::cluster_group cl = cg::this_cluster();
+  extern __shared__ double2 dyn[];   // a ring per warp; three sets of group sums; the vectors of this block's rows
+  __shared__ int current;
+  const int nw = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nb = static_cast<int>(cl.num_blocks()), rank = static_cast<int>(cl.block_rank());
+  char* ring = reinterpret_cast<char*>(dyn) + wid * kRingBytes;
+  double2* sums = dyn + nw * (kRingBytes / sizeof(double2));
+  const int cap = a.smem_rows;
+  double2* X = sums + 3 * kClusterAtoms / kGroup;
+  double2 *R = X + cap, *P = R + cap, *Q = P + cap, *D = Q + cap;
+  double* E = reinterpret_cast<double*>(D + cap);
+  int* cnt = reinterpret_cast<int*>(E + cap);
+  int flip = 0;
+  for (;;) {
+    if (rank == 0 && threadIdx.x == 0) {
+      const int t = atomicAdd(a.ticket, 1);
+      const int s = t < a.nsmall ? a.order[t] : -1;
+      for (int q = 0; q < nb; ++q) *cl.map_shared_rank(&current, static_cast<unsigned>(q)) = s;
+    }
+    cl.sync();
+    const int sy = current;
+    if (sy < 0) break;
+    const int i0 = d.sys[sy].begin, n = d.sys[sy].natoms;
+    const int groups = (n + kGroup - 1) / kGroup;
+    const int g0 = groups * rank / nb, g1 = groups * (rank + 1) / nb;
+    const int r0 = g0 * kGroup, m = max(0, min(g1 * kGroup, n) - r0), p0 = i0 + r0;
+    const int w0 = m * wid / nw, w1 = m * (wid + 1) / nw;   // this warp's rows (within the block's)
+    // hand the sums over this block's groups of `term` (a value per row) to every block
+    auto hand_over = [&](double2* set, auto term) {
+      for (int k0 = 0; k0 < m; k0 += blockDim.x) {
+        const int k = k0 + static_cast<int>(threadIdx.x);
+        double2 t = k < m ? term(k) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int o = 1; o < kGroup; o <<= 1) {
+          t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+          t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+        }
+        if (k < m && (k & (kGroup - 1)) == 0)
+          for (int q = 0; q < nb; ++q) cl.map_shared_rank(set, static_cast<unsigned>(q))[g0 + k / kGroup] = t;
+      }
+    };
+    auto total = [&](const double2* set) {   // in every thread
+      double v[2] = {0.0, 0.0};
+      for (int k = lane; k < groups; k += 32) {
+        v[0] += set[k].x;
+        v[1] += set[k].y;
+      }
+      const double t = warp_sums<2>(v);
+      return make_double2(__shfl_sync(0xffffffffu, t, 0), __shfl_sync(0xffffffffu, t, 16));
+    };
+    auto set_of = [&](int which) { return sums + which * (kClusterAtoms / kGroup); };
+    RowStream<true> rows;
+    for (int k = threadIdx.x; k < m; k += blockDim.x) {
+      X[k] = a.x[p0 + k];
+      E[k] = a.eta[p0 + k];
+      cnt[k] = d.nbr_cnt[p0 + k];
+    }
+    __syncthreads();
+    // ---- r = b - A x, d = M^-1 r; |b|^2 and r.d; first stop test
+    rows.start(d, p0 + w0, w1 - w0, cnt + w0, ring);
+    rows.run(d.amask, p0 + w0, a.x, Q + w0);
+    __syncthreads();
+    for (int k = threadIdx.x; k < m; k += blockDim.x) {
+      const double eta = E[k];
+      const double2 b = a.b[p0 + k], x = X[k], y = Q[k];
+      const double2 r = make_double2(b.x - (eta * x.x + y.x), b.y - (eta * x.y + y.y));
+      const double2 dd = make_double2(r.x / eta, r.y / eta);
+      R[k] = r;
+      D[k] = dd;
+      a.d[p0 + k] = dd;
+    }
+    hand_over(set_of(2), [&](int k) {
+      const double2 b = a.b[p0 + k];
+      return make_double2(b.x * b.x, b.y * b.y);
+    });
+    hand_over(set_of(flip), [&](int k) { return make_double2(R[k].x * D[k].x, R[k].y * D[k].y); });
+    rows.start(d, p0 + w0, w1 - w0, cnt + w0, ring);
+    cl.sync();
+    const double2 bb = total(set_of(2));
+    double2 sig = total(set_of(flip));
+    flip ^= 1;
+    const double bnorm_s = sqrt(bb.x), bnorm_t = sqrt(bb.y);
+    bool act_s = true, act_t = true, breakdown = false;
+    int it_s = 1, it_t = 1;
+    for (int it = 1; it < a.imax; ++it) {
+      act_s = act_s && (sqrt(sig.x) / bnorm_s > a.tol);
+      act_t = act_t && (sqrt(sig.y) / bnorm_t > a.tol);
+      if (!act_s && !act_t) break;
+      // ---- q = A d; d.q
+      rows.run(d.amask, p0 + w0, a.d, Q + w0);
+      __syncthreads();
+      hand_over(set_of(flip), [&](int k) {
+        const double eta = E[k];
+        const double2 dd = D[k];
+        double2 q = Q[k];
+        q.x += eta * dd.x; q.y += eta * dd.y;
+        Q[k] = q;
+        return make_double2(dd.x * q.x, dd.y * q.y);
+      });
+      rows.start(d, p0 + w0, w1 - w0, cnt + w0, ring);
+      cl.sync();
+      const double2 dq = total(set_of(flip));
+      flip ^= 1;
+      const double alpha_s = act_s ? sig.x / dq.x : 0.0;
+      const double alpha_t = act_t ? sig.y / dq.y : 0.0;
+      if (!(isfinite(alpha_s) && isfinite(alpha_t))) { breakdown = true; break; }
+      // ---- x += alpha d, r -= alpha q, p = M^-1 r; r.p
+      hand_over(set_of(flip), [&](int k) {
+        const double eta = E[k];
+        const double2 dd = D[k], q = Q[k];
+        double2 x = X[k], r = R[k];
+        x.x += alpha_s * dd.x; x.y += alpha_t * dd.y;
+        r.x -= alpha_s * q.x; r.y -= alpha_t * q.y;
+        const double2 p = make_double2(r.x / eta, r.y / eta);
+        X[k] = x;
+        R[k] = r;
+        P[k] = p;
+        return make_double2(r.x * p.x, r.y * p.y);
+      });
+      cl.sync();
+      const double2 rp = total(set_of(flip));
+      flip ^= 1;
+      const double beta_s = act_s ? rp.x / sig.x : 0.0, beta_t = act_t ? rp.y / sig.y : 0.0;
+      if (act_s) { sig.x = rp.x; it_s = it + 1; }
+      if (act_t) { sig.y = rp.y; it_t = it + 1; }
+      // ---- d = p + beta d (only for the right-hand sides still iterating)
+      for (int k = threadIdx.x; k < m; k += blockDim.x) {
+        const double2 p = P[k];
+        double2 dd = D[k];
+        if (act_s) dd.x = p.x + beta_s * dd.x;
+        if (act_t) dd.y = p.y + beta_t * dd.y;
+        D[k] = dd;
+        a.d[p0 + k] = dd;
+      }
+      cl.sync();
+    }
+    copy_wait<0>();   // the pieces of the pass that is not taken
+    __syncwarp();
+    // ---- calculate_Q: q = s - (sum s / sum t) t, the solution, the counts and residuals
+    __syncthreads();
+    hand_over(set_of(flip), [&](int k) { return X[k]; });
+    cl.sync();
+    const double2 sx = total(set_of(flip));
+    flip ^= 1;
+    const double c = sx.x / sx.y;
+    for (int k = threadIdx.x; k < m; k += blockDim.x) {
+      const double2 x = X[k];
+      a.x[p0 + k] = x;
+      if (a.write_q) {
+        const double q = x.x - c * x.y;
+        d.qr[p0 + k] = q;
+        d.q[d.cell_atoms[p0 + k]] = q;
+      }
+    }
+    if (rank == 0 && threadIdx.x == 0) {
+      const double rel_s = sqrt(sig.x) / bnorm_s, rel_t = sqrt(sig.y) / bnorm_t;
+      if (a.out_brk) a.out_brk[sy] = breakdown ? 1 : 0;
+      a.out_iters[2 * sy] = it_s;
+      a.out_iters[2 * sy + 1] = it_t;
+      a.out_rel[2 * sy] = rel_s;
+      a.out_rel[2 * sy + 1] = rel_t;
+      if (breakdown) atomicOr(d.status, ST_CG_BREAKDOWN);
+      if (!(rel_s <= a.tol && rel_t <= a.tol)) atomicOr(d.status, ST_CG_NOTCONV);
+    }
+  }
+}
+
+// Segmented Jacobi-PCG of the larger systems of a batch (more than kClusterAtoms atoms, too many for one cluster's share
+// of the GPU): all of them at once on one cooperative grid, the same algorithm (and the same
 // stopping rule per system, s and t separately) as the stock loop of fix qeq/reaxff (fix_qeq_reaxff_metal.cpp:89-123).
 // Rows of all systems are spread over all warps of the GPU, so one small system no longer runs on a single block.
 // Every dot product is a per-row term written to rb0/rb1; the warp that brings the last row of a system to a pass
@@ -1111,7 +1295,6 @@ __device__ inline bool arrive_last(SysCg* sc, int n, int cnt) {
 }
 
 __global__ void __launch_bounds__(256, 4) k_cg_seg(Dev d, CgArgs a) {
-  if (lists_failed(d)) return;
   cg::grid_group g = cg::this_grid();
   const int lane = threadIdx.x & 31;
   const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1150,6 +1333,7 @@ __global__ void __launch_bounds__(256, 4) k_cg_seg(Dev d, CgArgs a) {
         cur = s;
         cnt = 0;
       }
+      if (d.sys[s].natoms <= kClusterAtoms) continue;   // k_cg_cluster's (never live here)
       const double eta = a.eta[i];
       const double2 y = row_mv(d, i, eta, a.x);
       if (lane == 0) {
@@ -1281,6 +1465,7 @@ __global__ void __launch_bounds__(256, 4) k_cg_seg(Dev d, CgArgs a) {
 // ---- calculate_Q per system (warp per system): q = s - (sum s / sum t) t, the counts and residuals
   for (int s = gw; s < d.nsys; s += nw) {
     const SysInfo& si = d.sys[s];
+    if (si.natoms <= kClusterAtoms) continue;
     const double2 sum = sys_sum2(a.x, si.begin, si.natoms);
     const double u = sum.x / sum.y;
     if (a.write_q)

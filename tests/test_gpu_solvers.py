@@ -53,3 +53,70 @@ def test_static_solve_sizes_match_dense(n):
     assert rel.cpu().numpy().max() <= 1e-12 and it.cpu().numpy().max() < 500
     for got, ref in ((s, s_ref), (t, t_ref), (q, q_ref)):
         assert np.abs(got.cpu().numpy() - ref).max() <= 1e-8 * max(1.0, np.abs(ref).max())
+
+
+def _jittered(n, seed, spacing=2.3):
+    """n C/H/O atoms on random sites of a jittered cubic lattice (at least 20 A wide)."""
+    rng = np.random.default_rng(seed)
+    side = max(9, int(np.ceil(n ** (1.0 / 3.0))))
+    sites = rng.permutation(side ** 3)[:n]
+    x = np.stack([sites // side ** 2, sites // side % side, sites % side], axis=1) * spacing + rng.uniform(0.0, 0.7, size=(n, 3))
+    return {"name": "jitter%d" % n, "origin": np.zeros(3), "box": np.eye(3) * side * spacing, "periodic": np.ones(3, dtype=np.int32),
+            "x": x, "type": rng.integers(0, 3, size=n).astype(np.int32), "tag": np.arange(1, n + 1, dtype=np.int64)}
+
+
+@pytest.fixture(scope="module")
+def engine():
+    import rxcuda
+    from helpers import ffield_text
+    e = rxcuda.Engine(0)
+    e.set_forcefield(ffield_text())
+    e.set_control()
+    e.set_qeq(0.0, 10.0, 1e-12, 400)
+    yield e
+    e.close()
+
+
+@pytest.fixture(scope="module")
+def oracle():
+    from helpers import ffield_text
+    from oracle.oracle import COracle
+    return COracle(ffield_text(), shell=15.0)
+
+
+@pytest.mark.parametrize("n", [2, 7, 8, 9, 63, 128, 129, 1001, 4095, 4096, 4097, 6001])
+def test_charge_solve_sizes_match_oracle(engine, oracle, n):
+    """One system on both sides of a group of eight rows, of the blocks of a cluster (some own no row) and of the size where
+    all SMs take the solve, against the oracle's charges: 1e-10 e at tol 1e-12, as for the other sizes."""
+    s = _jittered(n, 7 + n)
+    engine.set_systems([s])
+    engine.qeq_reset()
+    got = engine.qeq_solve()
+    ref = oracle.qeq(s, tol=1e-12, imax=400)
+    assert np.abs(got["q"] - ref["q"]).max() <= 1e-10
+    # above 4096 atoms the solve restarts from an FP64 residual after every reduction by 1e6 (twice on the way to 1e-12),
+    # and a restarted CG needs up to two more iterations to regain its directions
+    assert np.abs(got["iters"][0] - ref["iters"]).max() <= (1 if n <= 4096 else 4)
+
+
+def test_mixed_batch_solves_alone_and_together(engine, oracle):
+    """Small systems (a cluster each) beside larger ones (all SMs): every small system's charges have the bits of its solve
+    alone, whatever cluster size the batch takes; the large ones match the oracle."""
+    ss = [_jittered(n, 90 + n) for n in (4500, 40, 700, 3, 4099, 2100)]
+    engine.set_systems(ss)
+    engine.qeq_reset()
+    both = engine.qeq_solve()
+    off = 0
+    for k, s in enumerate(ss):
+        n = len(s["type"])
+        if n <= 4096:
+            engine.set_systems([s])
+            engine.qeq_reset()
+            alone = engine.qeq_solve()
+            assert np.array_equal(alone["q"], both["q"][off:off + n]), n
+            assert np.array_equal(alone["iters"][0], both["iters"][k]), n
+        ref = oracle.qeq(s, tol=1e-12, imax=400)
+        assert np.abs(both["q"][off:off + n] - ref["q"]).max() <= 1e-10, n
+        off += n
+
+
