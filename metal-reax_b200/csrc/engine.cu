@@ -945,6 +945,11 @@ struct Context {
   // charges, so with tune.overlap it runs on `side` next to the row filter and the charge solve; the non-bonded pairs follow the charges on `stream`, and k_force_final joins both. Each branch writes its own arrays (fnb, vir_nb; bacc/bfn/fown; *_h; *_t, Tl), and
   // all join before the gathers, which add them in fixed order, so the schedule changes no result bit. With timing
   // on, every branch runs on `stream`, one after the other, so each phase is timed alone.
+  // at most one listed slot per bond (the tag-order end): half the slots bound the list; the warps go through it in
+  // strides, so that the many slots that are no central bond cost no blocks
+  unsigned torsion_blocks(int tpb) const {
+    return std::min(blocks((static_cast<long long>(na) * bcap + 1) / 2 * kLanes, tpb), static_cast<unsigned>(nsm * 2048 / tpb));
+  }
   void launch_bonded(const Dev& d) {
     const bool conc = !timing;
     cudaStream_t bs = conc ? side : stream, hs = conc ? side_h : stream, ts = conc ? side_t : stream;
@@ -966,13 +971,12 @@ struct Context {
     }
     tic(3, "bonded_terms");
     launches += 2;
-    k_bonded_atom<<<blocks(na, tune.tpb_atom), tune.tpb_atom, 0, bs>>>(d, dff, ctl);
+    k_bonded_atom<<<blocks(static_cast<long long>(na) * kLanes, tune.tpb_atom), tune.tpb_atom, 0, bs>>>(d, dff, ctl);
     k_hbond<<<blocks(static_cast<long long>(na) * 32, tune.tpb_hb), tune.tpb_hb, 0, hs>>>(d, dff, ctl);
     toc(3);
     tic(4, "torsion");
     ++launches;
-    // at most one listed slot per bond (the tag-order end): half the slots bound the list
-    k_torsion<<<blocks((static_cast<long long>(na) * bcap + 1) / 2, tune.tpb_atom), tune.tpb_atom, 0, ts>>>(d, dff, ctl);
+    k_torsion<<<torsion_blocks(tune.tpb_atom), tune.tpb_atom, 0, ts>>>(d, dff, ctl);
     toc(4);
     // the bonded gathers need the H-bond and torsion branches but no charge or non-bonded result: they stay on the
     // bonded branch, so only k_force_final follows the non-bonded pairs
@@ -1181,8 +1185,8 @@ struct Context {
     });
     pick(&tune.tpb_hb, {64, 128, 256}, [&](int t) { k_hbond<<<blocks(nw, t), t, 0, stream>>>(d, dff, ctl); });
     pick(&tune.tpb_atom, {32, 64, 128}, [&](int t) {
-      k_bonded_atom<<<blocks(na, t), t, 0, stream>>>(d, dff, ctl);
-      k_torsion<<<blocks((static_cast<long long>(na) * bcap + 1) / 2, t), t, 0, stream>>>(d, dff, ctl);
+      k_bonded_atom<<<blocks(static_cast<long long>(na) * kLanes, t), t, 0, stream>>>(d, dff, ctl);
+      k_torsion<<<torsion_blocks(t), t, 0, stream>>>(d, dff, ctl);
     });
     RXCU(cudaEventDestroy(a));
     RXCU(cudaEventDestroy(b));

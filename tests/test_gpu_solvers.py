@@ -120,3 +120,41 @@ def test_mixed_batch_solves_alone_and_together(engine, oracle):
         off += n
 
 
+
+
+@pytest.mark.parametrize("n,density", [(2, 0.02), (30, 1.0), (61, 3.0), (200, 2.0)])
+def test_bonded_terms_at_many_bonds_per_atom(engine, oracle, n, density):
+    """Angles and torsions shared by the lanes of an atom or central bond: from no bond to more bonds than lanes (dense random
+    carbon), against the oracle. FP64 terms, 1e-7 relative as in the parity tests; every decision identical."""
+    import systems
+    s = systems.random_carbon(n=n, density=density, seed=5 + n, dmin=0.95)
+    ref = oracle.single_point(s, np.zeros(n))
+    engine.set_systems([s])
+    engine.set_charges(np.zeros(n))
+    out = engine.compute(census=True)
+    terms = [0, 1, 2, 3, 4, 5, 6, 8, 9]
+    assert (np.abs(out["e"][0][terms] - ref["e"][terms]) / np.maximum(1.0, np.abs(ref["e"][terms]))).max() <= 1e-7
+    assert np.array_equal(out["census"], ref["census"])
+    scale = max(1.0, np.abs(ref["grad"]).max())
+    assert np.abs(out["grad"] - ref["grad"]).max() <= 1e-6 * scale
+    if density == 3.0:
+        assert ref["census"][0].max() > 8
+
+
+@pytest.mark.parametrize("n,density", [(2, 0.02), (30, 1.0), (61, 3.0), (200, 2.0)])
+def test_bonded_terms_at_many_bonds_per_atom(engine, oracle, n, density):
+    """Angles and torsions shared by the lanes of an atom or central bond: from no bond to more bonds than lanes (dense random
+    carbon), against the oracle. FP64 terms, 1e-7 relative as in the parity tests; every decision identical."""
+    import systems
+    s = systems.random_carbon(n=n, density=density, seed=5 + n, dmin=0.95)
+    ref = oracle.single_point(s, np.zeros(n))
+    engine.set_systems([s])
+    engine.set_charges(np.zeros(n))
+    out = engine.compute(census=True)
+    terms = [0, 1, 2, 3, 4, 5, 6, 8, 9]
+    assert (np.abs(out["e"][0][terms] - ref["e"][terms]) / np.maximum(1.0, np.abs(ref["e"][terms]))).max() <= 1e-7
+    assert np.array_equal(out["census"], ref["census"])
+    scale = max(1.0, np.abs(ref["grad"]).max())
+    assert np.abs(out["grad"] - ref["grad"]).max() <= 1e-6 * scale
+    if density == 3.0:
+        assert ref["census"][0].max() > 8
