@@ -234,7 +234,7 @@ int rx_md_targets(rx_context* ctx, const double* t_target, const int* active);
 
 /* Launch-shape tuning (no counterpart in the reference, whose Metal kernels use a fixed threadgroup of 64). All but
  * RX_TUNE_CG_BLOCKS_PER_SM leave every result bit unchanged. RX_TUNE_*_TPB: threads per block of a warp-per-atom kernel (64, 128, 256: atoms per
- * block x 32) or of the thread-per-atom bonded kernels (32, 64, 128); RX_TUNE_LONE_GRID_MIN: a context holding one
+ * block x 32) or of the bonded kernels (32, 64, 128); RX_TUNE_LONE_GRID_MIN: a context holding one
  * system of more atoms takes the single-system CG (all SMs on its rows, default 4096; a batch always takes the
  * segmented CG, so a system alone and in a batch give the same bits only below this size); RX_TUNE_OVERLAP: 1 (the
  * default) runs the bonded terms, which need no charge, concurrently with the charge solve, 0 after it;
