@@ -118,10 +118,9 @@ struct Context {
   std::vector<int> htype;
   std::vector<SysInfo> huser;   // systems as the caller gave them
   DBuf<SysInfo> sys;
-  DBuf<int> sys_of, type, cell_key, cell_key_sorted, cell_atoms, rank, atom_iota, cell_start, sys_flag;
+  DBuf<int> sys_of, type, cell_key, cell_key_sorted, cell_atoms, atom_iota, cell_start, sys_flag;
   DBuf<float4> xs;
-  DBuf<double4> xr;
-  DBuf<double> qr;
+  DBuf<double4> xr;   // cell-ordered positions, then the cell-ordered charges
   DBuf<long long> tag;
   DBuf<double4> x;
   DBuf<double> q;
@@ -154,12 +153,12 @@ struct Context {
   DBuf<double> epart;   // per (system, 256-atom chunk) partial sums of the energy terms and virial components
   int echunks = 1;
   // QEq
-  DBuf<double2> cg_x, cg_b, cg_r, cg_d, cg_p, cg_q, cg_s;
+  DBuf<double2> cg_x, cg_b, cg_r, cg_d, cg_p, cg_q;
   DBuf<float2> cg_df;
   DBuf<double> cg_eta, cg_part, s_hist, t_hist, cg_rel;
   DBuf<int> cg_iters, cg_nlive, cg_nref, cg_brk;
   DBuf<SysCg> cg_sys;
-  DBuf<int> cg_order, cg_ticket;   // systems of up to kClusterAtoms atoms, largest first; the clusters' counter
+  DBuf<int> cg_order;   // systems of up to kClusterAtoms atoms, largest first (not for a lone system)
   int n_small = 0, max_small = 0;
   long long rows_small = 0;
   DBuf<double2> cg_rb0, cg_rb1;
@@ -583,18 +582,16 @@ struct Context {
     cell_key.ensure(static_cast<size_t>(na));
     cell_key_sorted.ensure(static_cast<size_t>(na));
     cell_atoms.ensure(static_cast<size_t>(na));
-    rank.ensure(static_cast<size_t>(na));
     xs.ensure(static_cast<size_t>(na));
-    xr.ensure(static_cast<size_t>(na));
-    qr.ensure(static_cast<size_t>(na));
-    atom_iota.ensure(static_cast<size_t>(na));
+    xr.ensure(static_cast<size_t>(na) + (static_cast<size_t>(na) + 3) / 4);
+    atom_iota.ensure(2 * static_cast<size_t>(na));
     cell_start.ensure(static_cast<size_t>(ncell_total) + 1);
     {
-      std::vector<int> io(static_cast<size_t>(na));
-      for (int a = 0; a < na; ++a) io[static_cast<size_t>(a)] = a;
-      RXCU(cudaMemcpy(atom_iota.p, io.data(), sizeof(int) * na, cudaMemcpyHostToDevice));
-      // until the first rebuild (which every evaluation of a new layout starts with) the cell order is the atom order
-      RXCU(cudaMemcpy(rank.p, atom_iota.p, sizeof(int) * na, cudaMemcpyDeviceToDevice));
+      // the atom numbers, then the ranks: until the first rebuild (which every evaluation of a new layout starts with) the
+      // cell order is the atom order
+      std::vector<int> io(2 * static_cast<size_t>(na));
+      for (int a = 0; a < na; ++a) io[static_cast<size_t>(a)] = io[static_cast<size_t>(na) + a] = a;
+      RXCU(cudaMemcpy(atom_iota.p, io.data(), sizeof(int) * io.size(), cudaMemcpyHostToDevice));
     }
     key_bits = 1;
     while ((1LL << key_bits) <= ncell_total) ++key_bits;
@@ -637,7 +634,7 @@ struct Context {
     vir.ensure(n * kVir);
     vir_nb.ensure(n * kVir); vir_h.ensure(n * kVir); vir_t.ensure(n * kVir);
     fown_h.ensure(n); fown_t.ensure(n); fix_h.ensure(3 * n); pe_fix.ensure(n);
-    cg_x.ensure(n); cg_df.ensure(n); cg_b.ensure(n); cg_r.ensure(n); cg_d.ensure(n); cg_p.ensure(n); cg_q.ensure(n); cg_s.ensure(n); cg_eta.ensure(n);
+    cg_x.ensure(n); cg_df.ensure(n); cg_b.ensure(n); cg_r.ensure(n); cg_d.ensure(n); cg_p.ensure(n); cg_q.ensure(2 * n); cg_eta.ensure(n);
     cg_iters.ensure(2 * static_cast<size_t>(nsys)); cg_rel.ensure(2 * static_cast<size_t>(nsys));
     {
       std::vector<int> order;
@@ -652,11 +649,10 @@ struct Context {
       }
       n_small = static_cast<int>(order.size());
       std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return hsys[static_cast<size_t>(x)].natoms > hsys[static_cast<size_t>(y)].natoms; });
-      cg_order.ensure(order.size());
-      cg_ticket.ensure(1);
-      if (n_small > 0) RXCU(cudaMemcpy(cg_order.p, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice));
+      if (nsys > 1) cg_order.ensure(order.size());
+      if (nsys > 1 && n_small > 0) RXCU(cudaMemcpy(cg_order.p, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice));
     }
-    cg_sys.ensure(nsys); cg_rb0.ensure(n); cg_rb1.ensure(n); cg_nlive.ensure(2);
+    cg_sys.ensure(nsys); cg_rb0.ensure(n); cg_rb1.ensure(n); cg_nlive.ensure(3);
     cg_part.ensure(16 * static_cast<size_t>(std::max(nsm, 1)) * 32);
   }
 
@@ -686,7 +682,7 @@ struct Context {
   Dev dev() {
     Dev d{};
     d.na = na; d.nsys = nsys; d.sys = sys.p; d.sys_of = sys_of.p; d.x = x.p; d.type = type.p; d.tag = tag.p; d.q = q.p;
-    d.cell_key = cell_key.p; d.cell_atoms = cell_atoms.p; d.rank = rank.p; d.xr = xr.p; d.qr = qr.p; d.xs = xs.p; d.cell_start = cell_start.p; d.ncell_total = ncell_total;
+    d.cell_key = cell_key.p; d.cell_atoms = cell_atoms.p; d.rank = atom_iota.p + na; d.xr = xr.p; d.qr = reinterpret_cast<double*>(xr.p + na); d.xs = xs.p; d.cell_start = cell_start.p; d.ncell_total = ncell_total;
     d.ncap = ncap; d.nbr = nbr.p; d.nbr_cnt = nbr_cnt.p; d.hhi = hhi.p; d.hlo = hlo.p;
     d.vcap = vcap; d.vrow = vrow.p; d.vcnt = vcnt.p; d.xref = xref.p; d.sys_flag = sys_flag.p;
     d.rv2 = (ff.nonb_cut + skin) * (ff.nonb_cut + skin);
@@ -804,7 +800,7 @@ struct Context {
   CgArgs cg_args() {
     CgArgs a{};
     a.imax = qeq_imax; a.tol = qeq_tol;
-    a.x = cg_x.p; a.b = cg_b.p; a.r = cg_r.p; a.d = cg_d.p; a.p = cg_p.p; a.q = cg_q.p; a.s = cg_s.p; a.df = cg_df.p; a.eta = cg_eta.p; a.part = cg_part.p;
+    a.x = cg_x.p; a.b = cg_b.p; a.r = cg_r.p; a.d = cg_d.p; a.p = cg_p.p; a.q = cg_q.p; a.s = cg_q.p + na; a.df = cg_df.p; a.eta = cg_eta.p; a.part = cg_part.p;
     a.out_iters = cg_iters.p; a.out_rel = cg_rel.p; a.out_nref = cg_nref.p; a.out_brk = cg_brk.p; a.write_q = 1;
     return a;
   }
@@ -905,12 +901,12 @@ struct Context {
     }
     if (n_small > 0) {   // every system of up to kClusterAtoms atoms, alone or in a batch, by a cluster
       const int c = cluster_size();
-      a.order = cg_order.p; a.nsmall = n_small; a.ticket = cg_ticket.p;
+      a.order = nsys > 1 ? cg_order.p : nullptr; a.nsmall = n_small; a.ticket = cg_nlive.p + 2;
       a.smem_rows = cluster_rows(max_small, c);
       cudaLaunchAttribute at;
       cudaLaunchConfig_t cfg = cluster_config(c, &at);
       cfg.gridDim = dim3(static_cast<unsigned>(c * std::min(n_small, std::max(1, cluster_fit[c]))));
-      RXCU(cudaMemsetAsync(cg_ticket.p, 0, sizeof(int), stream));
+      RXCU(cudaMemsetAsync(a.ticket, 0, sizeof(int), stream));
       ++launches;
       RXCU(cudaLaunchKernelEx(&cfg, k_cg_cluster, d, a));
     }

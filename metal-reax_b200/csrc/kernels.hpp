@@ -46,7 +46,8 @@ struct CgArgs {
   int* out_nref;   // FP64 residual passes of the last single-system solve (may be null)
   int* out_brk;    // per system: 1 after a breakdown (a step length that is not finite)
   int write_q;     // 1: calculate_Q into the charges (the fix's solve); 0: solutions only
-  // cluster CG only: the systems it solves, largest first, their number, and the counter the clusters take them by
+  // cluster CG only: the systems it solves, largest first (null: the lone system), their number, and the counter the
+  // clusters take them by
   const int* order;
   int nsmall;
   int* ticket;

@@ -1107,7 +1107,7 @@ __global__ void __launch_bounds__(512, 2) k_cg_cluster(Dev d, CgArgs a) {
   for (;;) {
     if (rank == 0 && threadIdx.x == 0) {
       const int t = atomicAdd(a.ticket, 1);
-      const int s = t < a.nsmall ? a.order[t] : -1;
+      const int s = t < a.nsmall ? (a.order ? a.order[t] : t) : -1;
       for (int q = 0; q < nb; ++q) *cl.map_shared_rank(&current, static_cast<unsigned>(q)) = s;
     }
     cl.sync();

@@ -122,6 +122,24 @@ def test_mixed_batch_solves_alone_and_together(engine, oracle):
 
 
 
+def test_charge_solve_with_vectors_in_global_memory(engine):
+    """A system of more rows per block than shared memory holds (its vectors stay in global memory), against the segmented
+    FP64 solve of the same system. Both stop at a relative residual of 1e-10; diag(eta) + H has a condition number of a few
+    hundred, hence 1e-7 e."""
+    s = _jittered(200000, 3)
+    engine.set_qeq(0.0, 10.0, 1e-10, 400)
+    engine.set_systems([s])
+    engine.qeq_reset()
+    whole = engine.qeq_solve()
+    engine.set_tuning("lone_grid_min", 1 << 30)
+    engine.qeq_reset()
+    rows = engine.qeq_solve()
+    engine.set_tuning("lone_grid_min", 4096)
+    engine.set_qeq(0.0, 10.0, 1e-12, 400)
+    assert whole["rel"].max() <= 1e-10 and rows["rel"].max() <= 1e-10
+    assert np.abs(whole["q"] - rows["q"]).max() <= 1e-7
+
+
 @pytest.mark.parametrize("n,density", [(2, 0.02), (30, 1.0), (61, 3.0), (200, 2.0)])
 def test_bonded_terms_at_many_bonds_per_atom(engine, oracle, n, density):
     """Angles and torsions shared by the lanes of an atom or central bond: from no bond to more bonds than lanes (dense random
