@@ -1104,6 +1104,7 @@ __global__ void __launch_bounds__(512, 2) k_cg_cluster(Dev d, CgArgs a) {
   double* E = reinterpret_cast<double*>(D + cap);
   int* cnt = reinterpret_cast<int*>(E + cap);
   int flip = 0;
+  cl.sync();   // every block of the cluster has started: before that its shared memory must not be written
   for (;;) {
     if (rank == 0 && threadIdx.x == 0) {
       const int t = atomicAdd(a.ticket, 1);

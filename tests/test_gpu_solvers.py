@@ -120,6 +120,27 @@ def test_mixed_batch_solves_alone_and_together(engine, oracle):
         off += n
 
 
+def test_more_systems_than_clusters(engine, oracle):
+    """300 systems, more than the GPU holds clusters of even two blocks (148 SMs, one block each): every cluster takes several
+    and uses its shared memory again for each. Each system's charges have the bits of its solve alone; every 25th matches the
+    oracle to 1e-10 e at tol 1e-12, as for the other sizes."""
+    sizes = np.random.default_rng(11).integers(5, 201, size=300)
+    ss = [_jittered(int(n), 1000 + k) for k, n in enumerate(sizes)]
+    engine.set_systems(ss)
+    engine.qeq_reset()
+    both = engine.qeq_solve()
+    off = 0
+    for k, s in enumerate(ss):
+        n = len(s["type"])
+        engine.set_systems([s])
+        engine.qeq_reset()
+        alone = engine.qeq_solve()
+        assert np.array_equal(alone["q"], both["q"][off:off + n]), k
+        assert np.array_equal(alone["iters"][0], both["iters"][k]), k
+        if k % 25 == 0:
+            ref = oracle.qeq(s, tol=1e-12, imax=400)
+            assert np.abs(alone["q"] - ref["q"]).max() <= 1e-10, k
+        off += n
 
 
 def test_charge_solve_with_vectors_in_global_memory(engine):
