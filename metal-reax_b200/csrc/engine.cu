@@ -848,21 +848,22 @@ struct Context {
   // The cluster size with the shortest expected solve. An iteration of a system of n rows on c blocks takes about
   // kRowUs n / c + kMeetUs; the clusters share the systems, and none ends before the largest system's. Measured, us a
   // solve on 2, 4, 8, 16 blocks: 512 CHO systems of 64-1024 atoms 6925, 7235, 10885, 17918; 16 of 100-5000 (those up to
-  // 4096) 8: 2893, 16: 1542; one of 648 atoms 422, 250, 164, 116.
+  // 4096) 8: 2893, 16: 1542; one of 648 atoms 422, 250, 164, 116. 0 where the GPU holds no cluster of any size.
   int cluster_size() {
     constexpr double kRowUs = 0.25, kMeetUs = 4.0;
     int best = 0;
     double least = 0.0;
     for (int c : {16, 8, 4, 2}) {
       if (cluster_smem(max_small, c) > static_cast<size_t>(kCgSmem)) continue;
-      if (!cluster_fit[c]) {
-        RXCU(cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgSmem));
-        RXCU(cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      if (!cluster_fit[c]) {   // a size that the runtime refuses is one that does not fit
         cudaLaunchAttribute at;
         cudaLaunchConfig_t cfg = cluster_config(c, &at);
         cfg.dynamicSmemBytes = kCgSmem;
         int fits = 0;
-        if (cudaOccupancyMaxActiveClusters(&fits, k_cg_cluster, &cfg) != cudaSuccess) {
+        cudaError_t e = cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgSmem);
+        if (e == cudaSuccess && c > 8) e = cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fits, k_cg_cluster, &cfg);
+        if (e != cudaSuccess) {
           (void)cudaGetLastError();
           fits = 0;
         }
@@ -873,7 +874,6 @@ struct Context {
       const double t = std::max((kRowUs * rows_small / c + kMeetUs * n_small) / g, kRowUs * max_small / c + kMeetUs);
       if (!best || t < least) { best = c; least = t; }
     }
-    if (!best) throw Error(RX_ERR_CUDA, "no thread-block cluster of the charge solve fits the GPU");
     return best;
   }
 
@@ -899,8 +899,10 @@ struct Context {
       RXCU(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_cg_grid), dim3(grid), dim3(threads), args, smem, stream));
       return;
     }
-    if (n_small > 0) {   // every system of up to kClusterAtoms atoms, alone or in a batch, by a cluster
-      const int c = cluster_size();
+    // every system of up to kClusterAtoms atoms, alone or in a batch, by a cluster where the GPU holds one
+    const int c = n_small > 0 ? cluster_size() : 0;
+    a.cluster_max = c ? kClusterAtoms : 0;
+    if (c) {
       a.order = nsys > 1 ? cg_order.p : nullptr; a.nsmall = n_small; a.ticket = cg_nlive.p + 2;
       a.smem_rows = cluster_rows(max_small, c);
       cudaLaunchAttribute at;
@@ -910,7 +912,7 @@ struct Context {
       ++launches;
       RXCU(cudaLaunchKernelEx(&cfg, k_cg_cluster, d, a));
     }
-    if (n_small < nsys) {   // the larger systems of a batch: every row of every one on all SMs, per-system fixed-order sums
+    if (!c || n_small < nsys) {   // the others: every row of every one on all SMs, per-system fixed-order sums
       const int threads = 256;
       if (!seg_per_sm) RXCU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&seg_per_sm, k_cg_seg, threads, 0));
       int grid = std::max(1, std::min(seg_per_sm * nsm, (na + (threads / 32) - 1) / (threads / 32)));

@@ -52,6 +52,7 @@ struct CgArgs {
   int nsmall;
   int* ticket;
   // segmented CG only
+  int cluster_max; // systems of up to this many atoms are left to k_cg_cluster
   SysCg* sc;       // nsys
   double2* rb0;    // per-row dot-product terms (fixed-order per-system sums)
   double2* rb1;

@@ -1259,28 +1259,37 @@ __global__ void __launch_bounds__(512, 2) k_cg_cluster(Dev d, CgArgs a) {
   }
 }
 
-// Segmented Jacobi-PCG of the larger systems of a batch (more than kClusterAtoms atoms, too many for one cluster's share
-// of the GPU): all of them at once on one cooperative grid, the same algorithm (and the same
-// stopping rule per system, s and t separately) as the stock loop of fix qeq/reaxff (fix_qeq_reaxff_metal.cpp:89-123).
-// Rows of all systems are spread over all warps of the GPU, so one small system no longer runs on a single block.
+// Segmented Jacobi-PCG: every system that k_cg_cluster does not take (those of more than a.cluster_max atoms), all of them
+// at once on one cooperative grid, with the same algorithm and the same stopping rule per system, s and t separately, as the
+// stock loop of fix qeq/reaxff (fix_qeq_reaxff_metal.cpp:89-123). Their rows are spread over all warps of the GPU.
 // Every dot product is a per-row term written to rb0/rb1; the warp that brings the last row of a system to a pass
-// sums that system's terms in row order (lane-strided, then a butterfly), so a system's result depends only on its
-// own rows: it is bitwise the same alone and inside any batch. The iteration loop ends when no system is live; the
-// live count is kept per iteration parity so that no block can see it change before every block has read it.
+// sums that system's terms, so a system's result depends only on its own rows: it is bitwise the same alone and inside
+// any batch. Row products and sums take the order of k_cg_cluster (groups of eight rows, then a lane-strided sum of the
+// groups), so it is also bitwise the same whichever of the two kernels solves it. The iteration loop ends when no
+// system is live; the live count is kept per iteration parity so that no block can see it change before every block
+// has read it.
 __device__ inline double2 sys_sum2(const double2* v, int i0, int n) {
-  const int lane = threadIdx.x & 31;
-  double sx = 0.0, sy = 0.0;
-#pragma unroll 4
-  for (int k = lane; k < n; k += 32) {
-    const double2 t = __ldcg(v + i0 + k);
-    sx += t.x;
-    sy += t.y;
+  const int lane = threadIdx.x & 31, groups = (n + kGroup - 1) / kGroup;
+  double s[2] = {0.0, 0.0};
+  for (int g = lane; g < groups; g += 32) {
+    double2 t[kGroup];
+#pragma unroll
+    for (int k = 0; k < kGroup; ++k) {
+      const int row = g * kGroup + k;
+      t[k] = row < n ? __ldcg(v + i0 + row) : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int o = 1; o < kGroup; o <<= 1)   // the exchange of k_cg_cluster's hand-over, as its first lane sees it
+#pragma unroll
+      for (int k = 0; k < kGroup; k += 2 * o) {
+        t[k].x += t[k + o].x;
+        t[k].y += t[k + o].y;
+      }
+    s[0] += t[0].x;
+    s[1] += t[0].y;
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    sx += __shfl_xor_sync(0xffffffffu, sx, o);
-    sy += __shfl_xor_sync(0xffffffffu, sy, o);
-  }
-  return make_double2(sx, sy);
+  const double t = warp_sums<2>(s);
+  return make_double2(__shfl_sync(0xffffffffu, t, 0), __shfl_sync(0xffffffffu, t, 16));
 }
 
 // lane 0 counts cnt rows of the system in (after every lane's writes are fenced); true in every lane of the warp that
@@ -1334,7 +1343,7 @@ __global__ void __launch_bounds__(256, 4) k_cg_seg(Dev d, CgArgs a) {
         cur = s;
         cnt = 0;
       }
-      if (d.sys[s].natoms <= kClusterAtoms) continue;   // k_cg_cluster's (never live here)
+      if (d.sys[s].natoms <= a.cluster_max) continue;   // k_cg_cluster's (never live here)
       const double eta = a.eta[i];
       const double2 y = row_mv(d, i, eta, a.x);
       if (lane == 0) {
@@ -1466,7 +1475,7 @@ __global__ void __launch_bounds__(256, 4) k_cg_seg(Dev d, CgArgs a) {
 // ---- calculate_Q per system (warp per system): q = s - (sum s / sum t) t, the counts and residuals
   for (int s = gw; s < d.nsys; s += nw) {
     const SysInfo& si = d.sys[s];
-    if (si.natoms <= kClusterAtoms) continue;
+    if (si.natoms <= a.cluster_max) continue;
     const double2 sum = sys_sum2(a.x, si.begin, si.natoms);
     const double u = sum.x / sum.y;
     if (a.write_q)

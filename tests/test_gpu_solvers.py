@@ -1,6 +1,10 @@
 """The charge solvers at the sizes where their work split changes: fewer rows than warps, ragged blocks of rows, empty and
 long rows."""
 import ctypes
+import os
+import subprocess
+import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -141,6 +145,63 @@ def test_more_systems_than_clusters(engine, oracle):
             ref = oracle.qeq(s, tol=1e-12, imax=400)
             assert np.abs(alone["q"] - ref["q"]).max() <= 1e-10, k
         off += n
+
+
+# a stand-in for the runtime's occupancy query that refuses clusters of more than CLUSTERS_UP_TO blocks
+FEW_CLUSTERS = r"""
+#include <cuda_runtime_api.h>
+#include <dlfcn.h>
+#include <stdlib.h>
+cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void* f, const cudaLaunchConfig_t* c) {
+  typedef cudaError_t (*Query)(int*, const void*, const cudaLaunchConfig_t*);
+  for (unsigned k = 0; k < c->numAttrs; ++k)
+    if (c->attrs[k].id == cudaLaunchAttributeClusterDimension && (int)c->attrs[k].val.clusterDim.x > atoi(getenv("CLUSTERS_UP_TO")))
+      return cudaErrorInvalidClusterSize;
+  return ((Query)dlsym(dlopen("libcudart.so.12", RTLD_LAZY | RTLD_NOLOAD), "cudaOccupancyMaxActiveClusters"))(n, f, c);
+}
+"""
+
+
+def _with_few_clusters(tmp_path, limit, code):
+    """Runs `code` (this module's names at hand) in a process whose runtime refuses clusters of more than `limit` blocks;
+    returns the arrays that it puts into `out`."""
+    src, lib, got = tmp_path / "few.c", tmp_path / "few.so", tmp_path / "out.npz"
+    src.write_text("#define _GNU_SOURCE\n" + FEW_CLUSTERS)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-I/usr/local/cuda/include", str(src), "-o", str(lib), "-ldl"], check=True)
+    here = Path(__file__).resolve().parent
+    paths = [str(here), str(here.parent), str(here.parent / "metal-reax_b200")]
+    code = "import sys; sys.path[:0] = %r\nfrom test_gpu_solvers import *\nfrom test_gpu_solvers import _jittered, _random_csr\n" \
+           "out = {}\n%s\nnp.savez(%r, **out)\n" % (paths, code, str(got))
+    run = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, LD_PRELOAD=str(lib), CLUSTERS_UP_TO=str(limit)),
+                         capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]
+    return np.load(got)
+
+
+SOLVE_MIXED = """
+import rxcuda
+from helpers import ffield_text
+e = rxcuda.Engine(0)
+e.set_forcefield(ffield_text())
+e.set_control()
+e.set_qeq(0.0, 10.0, 1e-12, 400)
+for name, sizes in (("batch", (4500, 40, 700, 3, 4096, 2100)), ("lone", (1001,))):
+    e.set_systems([_jittered(n, 90 + n) for n in sizes])
+    e.qeq_reset()
+    got = e.qeq_solve()
+    out[name + "_q"], out[name + "_iters"], out[name + "_rel"] = got["q"], got["iters"], got["rel"]
+e.close()
+"""
+
+
+@pytest.mark.parametrize("limit", [0, 1, 8])
+def test_charge_solve_where_clusters_are_refused(tmp_path, limit):
+    """Where the GPU holds no cluster (or none of 16 blocks), the segmented solve takes the small systems too: the same
+    charges, counts and residuals to the last bit."""
+    few = _with_few_clusters(tmp_path, limit, SOLVE_MIXED)
+    all_ = _with_few_clusters(tmp_path, 16, SOLVE_MIXED)
+    for k in all_.files:
+        assert np.array_equal(few[k], all_[k]), k
 
 
 def test_charge_solve_with_vectors_in_global_memory(engine):
