@@ -222,6 +222,31 @@ def test_charge_solve_with_vectors_in_global_memory(engine):
     assert np.abs(whole["q"] - rows["q"]).max() <= 1e-7
 
 
+def test_bonded_time_grows_with_the_bonds(engine):
+    """Carbon of 14 and of 18 bonds on its most bonded atom (two and three bonds to a lane) has 2.3 times the angles; the bonded
+    terms take 1.5 times the time (they took 9 times when the lanes of a warp went through the exchange of the angles
+    apart). At most 4 times, so that other users' work on the machine does not matter."""
+    import systems
+    took, most = [], []
+    for density in (2.0, 3.0):
+        engine.set_systems([systems.random_carbon(n=4000, density=density, seed=5)])
+        engine.set_qeq(0.0, 10.0, 1e-6, 200)
+        engine.compute(qeq=True)
+        most.append(int(np.diff(engine.bonds()["start"]).max()))
+        engine.set_timing(True)
+        engine.compute(qeq=True)
+        runs = []
+        for _ in range(5):
+            before = engine.phase_times()["bonded_terms"]
+            engine.compute(qeq=True)
+            runs.append(engine.phase_times()["bonded_terms"] - before)
+        engine.set_timing(False)
+        took.append(min(runs))
+    engine.set_qeq(0.0, 10.0, 1e-12, 400)
+    assert most[0] <= 16 < most[1]
+    assert took[1] <= 4.0 * took[0], took
+
+
 @pytest.mark.parametrize("n,density", [(2, 0.02), (30, 1.0), (61, 3.0), (200, 2.0)])
 def test_bonded_terms_at_many_bonds_per_atom(engine, oracle, n, density):
     """Angles and torsions shared by the lanes of an atom or central bond: from no bond to more bonds than lanes (dense random
