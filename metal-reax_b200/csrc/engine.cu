@@ -117,6 +117,7 @@ struct Context {
   std::vector<long long> htag;
   std::vector<int> htype;
   std::vector<SysInfo> huser;   // systems as the caller gave them
+  std::vector<double> hvol;     // volume that the atoms of a system with a non-periodic direction take up (0: its cell's)
   DBuf<SysInfo> sys;
   DBuf<int> sys_of, type, cell_key, cell_key_sorted, cell_atoms, atom_iota, cell_start, sys_flag;
   DBuf<float4> xs;
@@ -420,6 +421,7 @@ struct Context {
     na = static_cast<int>(total);
     hsys.assign(static_cast<size_t>(nsys), SysInfo{});
     huser.clear();
+    hvol.assign(static_cast<size_t>(nsys), 0.0);
     hsys_of.resize(static_cast<size_t>(na));
     int begin = 0;
     for (int s = 0; s < nsys; ++s) {
@@ -877,6 +879,39 @@ struct Context {
     return best;
   }
 
+  // Whether the clusters of c blocks are the quicker way for the systems they can take: a lone system of thousands of
+  // atoms in long rows keeps all SMs busy and gains more from them than its grid barriers cost, and where the segmented solve
+  // runs for larger systems anyway, taking the small ones along costs it less than a launch of their own. The model of
+  // an iteration, us, from solves of 22-79 iterations (k_cg_cluster on 16 blocks: 13.1 at 648 atoms of water and 0.27 M
+  // entries, 34.3 at 4095 and 1.36 M, 18.9 at 1000 CHO atoms and 0.73 M, 39.5 at 2000 and 2.03 M; k_cg_seg: 19.7, 35.7,
+  // 22.3, 28.8, and 80 at four times 4000 atoms of water). Solves chosen by it, cluster and segmented, us: 1000 CHO
+  // atoms 1036, 1217; 4095 of water 1326, 1383; 3000 CHO atoms 2183, 1831; 2000 2896, 2144; six systems of 40 to 4500 atoms
+  // of water 3006, 2307; 16 CHO systems of 100-5000 4830, 6746. No result bit depends on the choice.
+  bool clusters_pay(int c) const {
+    auto cluster_us = [&](double n, double e) { return 9.6 + (0.027 * n + 2.1e-4 * e) / c; };
+    auto seg_us = [](double n, double e, double most) { return n > 0 ? 16.4 + 2.9e-3 * n + 2.6e-6 * e + 1e-3 * most : 0.0; };
+    const double ball = 4.0 / 3.0 * M_PI * ff.nonb_cut * ff.nonb_cut * ff.nonb_cut;
+    double sum = 0.0, longest = 0.0, n_large = 0.0, e_large = 0.0, n_all = 0.0, e_all = 0.0, most = 0.0;
+    for (int s = 0; s < nsys; ++s) {
+      const SysInfo& si = hsys[static_cast<size_t>(s)];
+      const double* L = si.L;
+      const double cell = L[0] * (L[4] * L[8] - L[5] * L[7]) + L[1] * (L[5] * L[6] - L[3] * L[8]) + L[2] * (L[3] * L[7] - L[4] * L[6]);
+      const double n = si.natoms, e = n * n * ball / (hvol[static_cast<size_t>(s)] > 0.0 ? hvol[static_cast<size_t>(s)] : cell);
+      n_all += n;
+      e_all += e;
+      most = std::max(most, n);
+      if (si.natoms > kClusterAtoms) {
+        n_large += n;
+        e_large += e;
+      } else {
+        sum += cluster_us(n, e);
+        longest = std::max(longest, cluster_us(n, e));
+      }
+    }
+    const double small = std::max(sum / std::min(n_small, cluster_fit[c]), longest);
+    return small + seg_us(n_large, e_large, most) <= seg_us(n_all, e_all, most);
+  }
+
   void launch_cg(const Dev& d, CgArgs a) {
     if (nsys == 1 && na > tune.lone_grid_min) {   // one large system: all SMs on its rows, block partials in block order
       const int units = tune.cg_per_sm > 0 ? std::min(tune.cg_per_sm, 4) : 4;
@@ -899,8 +934,9 @@ struct Context {
       RXCU(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_cg_grid), dim3(grid), dim3(threads), args, smem, stream));
       return;
     }
-    // every system of up to kClusterAtoms atoms, alone or in a batch, by a cluster where the GPU holds one
-    const int c = n_small > 0 ? cluster_size() : 0;
+    // the systems of up to kClusterAtoms atoms, alone or in a batch, by a cluster each where the GPU holds one and it pays
+    int c = n_small > 0 ? cluster_size() : 0;
+    if (c && !clusters_pay(c)) c = 0;
     a.cluster_max = c ? kClusterAtoms : 0;
     if (c) {
       a.order = nsys > 1 ? cg_order.p : nullptr; a.nsmall = n_small; a.ticket = cg_nlive.p + 2;
@@ -1240,6 +1276,7 @@ struct Context {
         for (int c2 = 0; c2 < 3; ++c2) si.origin[c2] = u.origin[c2];
         for (int c2 = 0; c2 < 9; ++c2) si.L[c2] = u.L[c2];
         const double reach = ff.nonb_cut + skin + kNpPad;
+        hvol[static_cast<size_t>(sy)] = det;
         for (int k = 0; k < 3; ++k) {
           if (u.per[k]) continue;
           double fmin = HUGE_VAL, fmax = -HUGE_VAL;
@@ -1253,6 +1290,7 @@ struct Context {
           const double m = reach / hk[k];                 // margin in the caller's fractional units
           const double scale = (fmax - fmin) + 2.0 * m;   // new length along k in units of the caller's vector
           const double t = fmin - m;
+          hvol[static_cast<size_t>(sy)] *= fmax - fmin + ff.nonb_cut / hk[k];
           for (int c2 = 0; c2 < 3; ++c2) {
             si.origin[c2] += t * L[3 * k + c2];
             si.L[3 * k + c2] = scale * L[3 * k + c2];
@@ -1683,7 +1721,9 @@ struct Context {
       og.ensure(static_cast<size_t>(old_na));
       RXCU(cudaMemcpy(og.p, grad.p, sizeof(double4) * old_na, cudaMemcpyDeviceToDevice));
     }
+    const std::vector<double> old_vol = hvol;
     set_systems(ns, nat.data(), org.data(), bx.data(), per.data(), ty.data(), tg.data());
+    for (int k = 0; k < nkeep; ++k) hvol[static_cast<size_t>(k)] = old_vol[static_cast<size_t>(keep[k])];
     if (nadd > 0) {   // new systems start with cold charge histories
       RXCU(cudaMemset(s_hist.p + 4 * nkept_atoms, 0, sizeof(double) * 4 * nadd));
       RXCU(cudaMemset(t_hist.p + 4 * nkept_atoms, 0, sizeof(double) * 4 * nadd));

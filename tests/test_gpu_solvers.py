@@ -175,7 +175,8 @@ def _with_few_clusters(tmp_path, limit, code):
     run = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, LD_PRELOAD=str(lib), CLUSTERS_UP_TO=str(limit)),
                          capture_output=True, text=True, timeout=300)
     assert run.returncode == 0, run.stderr[-2000:]
-    return np.load(got)
+    with np.load(got) as z:
+        return {k: z[k] for k in z.files}
 
 
 SOLVE_MIXED = """
@@ -200,8 +201,41 @@ def test_charge_solve_where_clusters_are_refused(tmp_path, limit):
     charges, counts and residuals to the last bit."""
     few = _with_few_clusters(tmp_path, limit, SOLVE_MIXED)
     all_ = _with_few_clusters(tmp_path, 16, SOLVE_MIXED)
-    for k in all_.files:
+    for k in all_:
         assert np.array_equal(few[k], all_[k]), k
+
+
+TIME_SOLVES = """
+import time
+import rxcuda
+import systems
+from helpers import ffield_text
+e = rxcuda.Engine(0)
+e.set_forcefield(ffield_text())
+e.set_control()
+e.set_qeq(0.0, 10.0, 1e-6, 200)
+dense = systems.serving_request(0, seed=1, nmin=2000, nmax=2000)[0]
+for name, ss in (("dense", [dense]), ("mixed", [systems.water_box(m) for m in (12, 3, 6, 5, 12, 9)])):
+    e.set_systems(ss)
+    e.qeq_solve()
+    took = []
+    for _ in range(9):
+        e.qeq_reset()
+        t = time.perf_counter()
+        e.qeq_solve()
+        took.append(time.perf_counter() - t)
+    out[name] = min(took)
+e.close()
+"""
+
+
+def test_charge_solve_takes_the_quicker_kernel(tmp_path):
+    """A lone system of 2000 atoms in rows of 1000 entries, and small systems beside larger ones (water of 81 to 5184 atoms): the
+    clusters take 1.3 times as long there as the segmented solve, so they are not taken. At most 1.2 times the solve
+    without clusters, for the noise of the machine."""
+    rule, without = (_with_few_clusters(tmp_path, limit, TIME_SOLVES) for limit in (16, 0))
+    for k in rule:
+        assert rule[k] <= 1.2 * without[k], (k, float(rule[k]), float(without[k]))
 
 
 def test_charge_solve_with_vectors_in_global_memory(engine):
