@@ -230,6 +230,9 @@ __device__ inline bool lists_failed(const Dev& d) {
   return (*reinterpret_cast<volatile const int*>(d.status) &
           (ST_NBR_OVERFLOW | ST_NEAR_OVERFLOW | ST_BOND_OVERFLOW | ST_SHIFT_RANGE | ST_VERLET_OVERFLOW | ST_ACC_OVERFLOW)) != 0;
 }
+// The same for a whole warp (all of whose lanes call it): the other branch of the evaluation may set the flags meanwhile, and
+// lanes that read them differently would leave some of the warp waiting in the exchanges that follow.
+__device__ inline bool warp_lists_failed(const Dev& d) { return __any_sync(0xffffffffu, lists_failed(d)); }
 
 // Virial of an interaction cluster, sum over its atoms of x_a f_b = -x_a g_b, taken with positions P relative to the
 // cluster's own atom (every term is translation invariant, so its gradients sum to zero and the origin drops out).

@@ -67,7 +67,7 @@ __device__ inline void add3(double4& a, double s, const double* v) { a.x += s * 
 // One warp per atom over its neighbor row: entries within bond_cut whose uncorrected bond order passes bo_cut
 // (terms::bo_prime, terms.hpp:50-56; gate src/cpu/bonded.cpp:130) become bond slots, in row order.
 __global__ void k_bonds(Dev d, DevFF ff, DevCtl ctl) {
-  if (lists_failed(d)) return;
+  if (warp_lists_failed(d)) return;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= d.na) return;
@@ -308,7 +308,7 @@ struct AngleOut {   // what one angle adds: Cdbo, CdDelta and gradient of its fi
 };
 
 __global__ void __launch_bounds__(128, 3) k_bonded_atom(Dev d, DevFF ff, DevCtl ctl) {
-  if (lists_failed(d)) return;
+  if (warp_lists_failed(d)) return;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int g = threadIdx.x & (kLanes - 1);
   const int lane0 = threadIdx.x & 31 & ~(kLanes - 1);   // the first of this atom's lanes
@@ -692,7 +692,7 @@ __device__ inline bool hbond_triple(const DevFF& ff, const HbDonor& dn, int tj, 
 // gradient of the donor bond are reduced over the warp in fixed order (the donor's share goes to j's slot for the
 // donor to gather); the acceptor's gradient is added to its fixed-point accumulator (zeroed by k_nbr_check).
 __global__ void __launch_bounds__(256, 3) k_hbond(Dev d, DevFF ff, DevCtl ctl) {
-  if (lists_failed(d)) return;
+  if (warp_lists_failed(d)) return;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= d.na) return;
@@ -816,7 +816,7 @@ struct TorsionOut {   // gradient on i and Cdbo of i-j, gradient on l and Cdbo o
 };
 
 __global__ void __launch_bounds__(128, 3) k_torsion(Dev d, DevFF ff, DevCtl ctl) {
-  if (lists_failed(d)) return;
+  if (warp_lists_failed(d)) return;
   const int g = threadIdx.x & (kLanes - 1);
   const int lane0 = threadIdx.x & 31 & ~(kLanes - 1);   // the first of this central bond's lanes
   const int listed = *d.tor_n;

@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(256) k_pairs(Dev d, DevFF ff, QeqParams qp) {
   const int warp = gid >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= d.na) return;
-  if (lists_failed(d)) {   // the evaluation is repeated: empty rows keep the kernels after this one inside the lists
+  if (warp_lists_failed(d)) {   // the evaluation is repeated: empty rows keep the kernels after this one inside the lists
     if (lane == 0) d.nbr_cnt[warp] = 0;
     return;
   }
@@ -423,7 +423,7 @@ __device__ __forceinline__ float nb_pair_terms(const DevFF& ff, int ti, int tj, 
 // at i if it is owned-owned with j > i, or a periodic image with tag_i < tag_j or, for an image of i itself, the
 // positive direction; each counted entry contributes its full pair energy (terms::nonbonded_pair, terms.hpp:282-323).
 __global__ void k_nonbonded(Dev d, DevFF ff) {
-  if (lists_failed(d)) return;
+  if (warp_lists_failed(d)) return;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= d.na) return;
@@ -508,7 +508,7 @@ __global__ void k_nonbonded(Dev d, DevFF ff) {
 // batch of 32 has a pair to compute. The pair virial goes whole to the owner; the per-atom split of energies and
 // virials (RX_COMPUTE_PERATOM) takes k_nonbonded instead.
 __global__ void __launch_bounds__(256) k_nonbonded_half(Dev d, DevFF ff) {
-  if (lists_failed(d)) return;
+  if (warp_lists_failed(d)) return;
   __shared__ unsigned queue[8][64];
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
@@ -633,7 +633,7 @@ __global__ void k_count_pairs(Dev d) {
 // energy takes the owner-computes counted entries, as k_nonbonded. Adds to the non-bonded branch's arrays (the same
 // stream, after k_nonbonded).
 __global__ void k_acks2(Dev d, DevFF ff, const double* s_kin) {
-  if (lists_failed(d)) return;
+  if (warp_lists_failed(d)) return;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= d.na) return;

@@ -25,3 +25,14 @@ def test_cluster_meets_before_its_first_remote_access():
     for f, n, body in remote:
         meet = body.find("cl.sync()")
         assert 0 <= meet < body.find("map_shared_rank"), "%s: %s reaches into another block before the cluster has met" % (f, n)
+
+
+def test_warps_leave_after_a_list_overflow_together():
+    """The overflow flags may be set while a kernel runs (by the other branch of the evaluation). A kernel whose lanes exchange
+    values takes one decision a warp: a lane that left alone would be missed by the others."""
+    seen = set()
+    for f, n, body in kernels():
+        if "lists_failed(d)" in body and re.search(r"_sync\(|warp_sum|lanes_sum", body.replace("__threadfence", "")):
+            seen.add(n)
+            assert not re.search(r"(?<!warp_)lists_failed\(d\)", body), "%s: %s leaves lane by lane" % (f, n)
+    assert seen >= {"k_pairs", "k_nonbonded_half", "k_bonds", "k_bonded_atom", "k_hbond", "k_torsion"}
