@@ -24,7 +24,7 @@ namespace {
 constexpr int kStaticMaxAtoms = RX_QEQ_STATIC_MAX_ATOMS;
 constexpr int kMaxDevices = 64;
 constexpr int kStaticThreads = 1024;
-constexpr int kStaticCluster = 16;   // blocks of the solve's cluster (8, the portable size, where 16 cannot be had)
+constexpr int kStaticCluster = 16;   // blocks of the solve's cluster (half as many, and so on, where they cannot be had)
 
 }  // namespace
 
@@ -260,13 +260,19 @@ extern "C" int rx_qeq_solve_static(int n, const int* row_start, const int* col, 
       cudaError_t e = cudaGetSymbolAddress(&ptr, rx_qeq_static_scratch);
       cudaFuncAttributes fa;
       if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_cg_csr_static);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cg_csr_static, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e == cudaSuccess) {
-        cudaLaunchAttribute at;
-        cudaLaunchConfig_t cfg = static_launch(kStaticCluster, nullptr, &at);
-        int fits = 0;
-        e = cudaOccupancyMaxActiveClusters(&fits, k_cg_csr_static, &cfg);
-        g_cluster[dev] = fits > 0 ? kStaticCluster : 8;
+      if (e == cudaSuccess) {   // a size that the runtime refuses is one that does not fit; what it leaves behind is cleared
+        const bool clean = cudaPeekAtLastError() == cudaSuccess;
+        int c = kStaticCluster;
+        for (; c > 1; c /= 2) {
+          cudaLaunchAttribute at;
+          cudaLaunchConfig_t cfg = static_launch(c, nullptr, &at);
+          int fits = 0;
+          cudaError_t q = c > 8 ? cudaFuncSetAttribute(k_cg_csr_static, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : cudaSuccess;
+          if (q == cudaSuccess) q = cudaOccupancyMaxActiveClusters(&fits, k_cg_csr_static, &cfg);
+          if (q != cudaSuccess && clean) (void)cudaGetLastError();
+          if (q == cudaSuccess && fits > 0) break;
+        }
+        g_cluster[dev] = c;
       }
       if (e != cudaSuccess) {
         char m[200];

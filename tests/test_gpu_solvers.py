@@ -205,6 +205,36 @@ def test_charge_solve_where_clusters_are_refused(tmp_path, limit):
         assert np.array_equal(few[k], all_[k]), k
 
 
+SOLVE_STATIC = """
+import torch
+import rxcuda
+lib, err = rxcuda.load(), ctypes.create_string_buffer(256)
+H, rs, col, val, eta, chi = _random_csr(300, 5)
+up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+rs, col, val, eta, chi = up(rs), up(col), up(val), up(eta), up(chi)
+s, t, q = (torch.zeros(300, dtype=torch.float64, device="cuda") for _ in range(3))
+it, rel = torch.zeros(2, dtype=torch.int32, device="cuda"), torch.zeros(2, dtype=torch.float64, device="cuda")
+rc = lib.rx_qeq_solve_static(300, *(a.data_ptr() for a in (rs, col, val, eta, chi, s, t, q)), 1e-12, 500, it.data_ptr(),
+                             rel.data_ptr(), torch.cuda.current_stream().cuda_stream, err, 256)
+assert rc == 0, err.value
+torch.cuda.synchronize()
+out["q"], out["rel"] = q.cpu().numpy(), rel.cpu().numpy()
+"""
+
+
+@pytest.mark.parametrize("limit", [0, 2, 8])
+def test_static_solve_where_clusters_are_refused(tmp_path, limit):
+    """Where the runtime refuses 16 blocks the solve takes the largest cluster that there is, down to one block. The blocks' sums
+    are added in another order, hence the bound of the test above: 1e-8 of the largest charge at tol 1e-12."""
+    few = _with_few_clusters(tmp_path, limit, SOLVE_STATIC)
+    H, _, _, _, eta, chi = _random_csr(300, 5)
+    A = np.diag(eta) + H
+    s_ref, t_ref = np.linalg.solve(A, -chi), np.linalg.solve(A, -np.ones(300))
+    q_ref = s_ref - s_ref.sum() / t_ref.sum() * t_ref
+    assert few["rel"].max() <= 1e-12
+    assert np.abs(few["q"] - q_ref).max() <= 1e-8 * max(1.0, np.abs(q_ref).max())
+
+
 TIME_SOLVES = """
 import time
 import rxcuda
