@@ -24,11 +24,13 @@ namespace {
 constexpr int kStaticMaxAtoms = RX_QEQ_STATIC_MAX_ATOMS;
 constexpr int kMaxDevices = 64;
 constexpr int kStaticThreads = 1024;
+constexpr int kOneBlockThreads = 512;
+constexpr int kOneBlockAtoms = 112;   // systems of up to this many atoms are one block's
 constexpr int kStaticCluster = 16;   // blocks of the solve's cluster (half as many, and so on, where they cannot be had)
 
 }  // namespace
 
-// CG work vectors r, d and q for the s and t systems (6 of the 8 doubles per atom; 2 MiB for 32768 atoms).
+// CG work vectors r, d, q and, for one block, M^-1 r for the s and t systems (8 doubles per atom; 2 MiB for 32768 atoms).
 static __device__ __align__(256) double rx_qeq_static_scratch[static_cast<size_t>(kStaticMaxAtoms) * 8];
 
 namespace {
@@ -85,6 +87,11 @@ __device__ inline double2 csr_row_mv(int i, const int* __restrict__ rs, const in
 // the cluster owns the rows [r n / C, (r + 1) n / C). A cluster's hardware barrier and its blocks' shared memory carry
 // the dot products, so the launch is a plain one: no grid-wide barrier whose workspace the driver would have to
 // provide. Only the search direction d is read by other blocks; r and q = A d stay with their block.
+//
+// kOneBlock: the system is one block's, which meets at its own barrier and keeps M^-1 r (a division in FP64 takes longer than the
+// rest of a small system's vector update). An iteration of one block, of clusters, us: 24 atoms of water 5.3, 7.9; 64 6.2,
+// 8.1; 96 7.5, 8.0; 129 9.8, 9.7; 160 11.6, 9.6.
+template <bool kOneBlock>
 __global__ void __launch_bounds__(kStaticThreads) k_cg_csr_static(int n, const int* rs, const int* col, const double* val,
                                                                   const double* eta, const double* chi, double* s_io, double* t_io,
                                                                   double* q_out, double tol, int imax, int* iters, double* rel,
@@ -93,11 +100,16 @@ __global__ void __launch_bounds__(kStaticThreads) k_cg_csr_static(int n, const i
   double2* r = reinterpret_cast<double2*>(scratch);
   double2* d = r + n;
   double2* qv = d + n;
+  double2* p = qv + n;
   __shared__ double sh[32 * 4];
   __shared__ double part[2][4];   // this block's partial sums (two sets in turn: one may still be read by a slower block)
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int nb = static_cast<int>(cl.num_blocks()), rank = static_cast<int>(cl.block_rank());
   const int r0 = static_cast<int>(static_cast<long long>(n) * rank / nb), r1 = static_cast<int>(static_cast<long long>(n) * (rank + 1) / nb);
+  auto meet = [&]() {
+    if (kOneBlock) __syncthreads();
+    else cl.sync();
+  };
   int flip = 0;
   // sums over the cluster: warps, then the block's warps in order, then the blocks in order (the same in every block)
   auto reduce = [&](double* v, int nv) {
@@ -112,9 +124,13 @@ __global__ void __launch_bounds__(kStaticThreads) k_cg_csr_static(int n, const i
       for (int w = 0; w < nw; ++w) t += sh[w * 4 + threadIdx.x];
       part[flip][threadIdx.x] = t;
     }
-    cl.sync();
+    meet();
     // lane b of every warp fetches block b's partials; the sums run over the blocks in order
     for (int k = 0; k < nv; ++k) {
+      if (kOneBlock) {
+        v[k] = part[flip][k];
+        continue;
+      }
       const double mine = lane < nb ? cl.map_shared_rank(&part[flip][0], static_cast<unsigned>(lane))[k] : 0.0;
       double t = 0.0;
       for (int b = 0; b < nb; ++b) t += __shfl_sync(0xffffffffu, mine, b);
@@ -124,7 +140,7 @@ __global__ void __launch_bounds__(kStaticThreads) k_cg_csr_static(int n, const i
   };
   // the current iterate lives in d for the first product: copy the caller's guesses there
   for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) d[i] = make_double2(s_io[i], t_io[i]);
-  cl.sync();
+  meet();
   double loc[4] = {0.0, 0.0, 0.0, 0.0};
   for (int i = r0 + wid; i < r1; i += nw) {
     const double e = eta[i];
@@ -143,7 +159,7 @@ __global__ void __launch_bounds__(kStaticThreads) k_cg_csr_static(int n, const i
     const double e = eta[i];
     d[i] = make_double2(rr.x / e, rr.y / e);
   }
-  cl.sync();
+  meet();
   const double bnorm_s = sqrt(loc[0]), bnorm_t = sqrt(loc[1]);
   double sig_s = loc[2], sig_t = loc[3];
   bool act_s = true, act_t = true, broke_s = false, broke_t = false;
@@ -178,7 +194,9 @@ __global__ void __launch_bounds__(kStaticThreads) k_cg_csr_static(int n, const i
       rr.x -= alpha_s * qq.x; rr.y -= alpha_t * qq.y;
       r[i] = rr;
       const double e = eta[i];
-      loc[0] += rr.x * (rr.x / e); loc[1] += rr.y * (rr.y / e);
+      const double2 pp = make_double2(rr.x / e, rr.y / e);
+      if (kOneBlock) p[i] = pp;
+      loc[0] += rr.x * pp.x; loc[1] += rr.y * pp.y;
     }
     reduce(loc, 2);
     const double beta_s = act_s ? loc[0] / sig_s : 0.0;
@@ -186,14 +204,19 @@ __global__ void __launch_bounds__(kStaticThreads) k_cg_csr_static(int n, const i
     if (act_s) { sig_s = loc[0]; it_s = it + 1; }
     if (act_t) { sig_t = loc[1]; it_t = it + 1; }
     for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
-      const double2 rr = r[i];
-      const double e = eta[i];
-      double2 dd = d[i];
-      if (act_s) dd.x = rr.x / e + beta_s * dd.x;
-      if (act_t) dd.y = rr.y / e + beta_t * dd.y;
+      double2 pp, dd = d[i];
+      if (kOneBlock) {
+        pp = p[i];
+      } else {
+        const double2 rr = r[i];
+        const double e = eta[i];
+        pp = make_double2(rr.x / e, rr.y / e);
+      }
+      if (act_s) dd.x = pp.x + beta_s * dd.x;
+      if (act_t) dd.y = pp.y + beta_t * dd.y;
       d[i] = dd;
     }
-    cl.sync();
+    meet();
   }
   loc[0] = loc[1] = 0.0;
   for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) { loc[0] += s_io[i]; loc[1] += t_io[i]; }
@@ -204,20 +227,20 @@ __global__ void __launch_bounds__(kStaticThreads) k_cg_csr_static(int n, const i
     if (iters) { iters[0] = broke_s ? -1 : it_s; iters[1] = broke_t ? -1 : it_t; }
     if (rel) { rel[0] = sqrt(sig_s) / bnorm_s; rel[1] = sqrt(sig_t) / bnorm_t; }
   }
-  cl.sync();   // no block leaves while another may still read its partial sums
+  meet();   // no block leaves while another may still read its partial sums
 }
 
 cudaLaunchConfig_t static_launch(int cluster, cudaStream_t stream, cudaLaunchAttribute* at) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(cluster));
-  cfg.blockDim = dim3(kStaticThreads);
+  cfg.blockDim = dim3(cluster > 1 ? kStaticThreads : kOneBlockThreads);
   cfg.stream = stream;
   at->id = cudaLaunchAttributeClusterDimension;
   at->val.clusterDim.x = static_cast<unsigned>(cluster);
   at->val.clusterDim.y = 1;
   at->val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
   return cfg;
 }
 
@@ -259,7 +282,8 @@ extern "C" int rx_qeq_solve_static(int n, const int* row_start, const int* col, 
       void* ptr = nullptr;
       cudaError_t e = cudaGetSymbolAddress(&ptr, rx_qeq_static_scratch);
       cudaFuncAttributes fa;
-      if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_cg_csr_static);
+      if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_cg_csr_static<true>);
+      if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_cg_csr_static<false>);
       if (e == cudaSuccess) {   // a size that the runtime refuses is one that does not fit; what it leaves behind is cleared
         const bool clean = cudaPeekAtLastError() == cudaSuccess;
         int c = kStaticCluster;
@@ -267,8 +291,8 @@ extern "C" int rx_qeq_solve_static(int n, const int* row_start, const int* col, 
           cudaLaunchAttribute at;
           cudaLaunchConfig_t cfg = static_launch(c, nullptr, &at);
           int fits = 0;
-          cudaError_t q = c > 8 ? cudaFuncSetAttribute(k_cg_csr_static, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : cudaSuccess;
-          if (q == cudaSuccess) q = cudaOccupancyMaxActiveClusters(&fits, k_cg_csr_static, &cfg);
+          cudaError_t q = c > 8 ? cudaFuncSetAttribute(k_cg_csr_static<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : cudaSuccess;
+          if (q == cudaSuccess) q = cudaOccupancyMaxActiveClusters(&fits, k_cg_csr_static<false>, &cfg);
           if (q != cudaSuccess && clean) (void)cudaGetLastError();
           if (q == cudaSuccess && fits > 0) break;
         }
@@ -293,8 +317,9 @@ extern "C" int rx_qeq_solve_static(int n, const int* row_start, const int* col, 
   // no more blocks than have a row for every warp: a small system's barriers cost more than its rows
   const int rows_per_block = kStaticThreads / 32;
   while (cluster > 1 && (cluster / 2) * rows_per_block >= n) cluster /= 2;
+  if (n <= kOneBlockAtoms) cluster = 1;
   const cudaLaunchConfig_t cfg = static_launch(cluster, static_cast<cudaStream_t>(stream), &at);
-  (void)cudaLaunchKernelEx(&cfg, k_cg_csr_static, n, row_start, col, val, eta, chi, s, t, q, tol, imax, iters, rel, scratch);
+  (void)cudaLaunchKernelEx(&cfg, cluster > 1 ? k_cg_csr_static<false> : k_cg_csr_static<true>, n, row_start, col, val, eta, chi, s, t, q, tol, imax, iters, rel, scratch);
   // peek, not get: the error state is left as it is for the caller (an error still pending from earlier work on this
   // thread is therefore reported here too)
   const cudaError_t e = cudaPeekAtLastError();

@@ -28,9 +28,9 @@ def _random_csr(n, seed):
     return H, rs, cols.astype(np.int32), H[rows, cols], eta, rng.uniform(-5.0, 5.0, size=n)
 
 
-@pytest.mark.parametrize("n", [2, 3, 15, 16, 17, 64, 129, 255, 257, 1000, 1999])
+@pytest.mark.parametrize("n", [2, 3, 15, 16, 17, 31, 32, 33, 64, 65, 111, 112, 113, 127, 128, 129, 255, 256, 257, 1000, 1999])
 def test_static_solve_sizes_match_dense(n):
-    """Sizes on both sides of a block's 16 rows and of the cluster's halvings, against the dense FP64 solution. At tol 1e-12
+    """Sizes on both sides of a block's rows a warp, of the change from one block (112) to a cluster and of the cluster's halvings, against the dense FP64 solution. At tol 1e-12
     the residual bounds the error: |x - x*| <= cond * tol * |x|; the matrices are diagonally dominant by a factor that keeps
     cond below 1e3, hence 1e-8 of the largest charge."""
     import torch
@@ -233,6 +233,41 @@ def test_static_solve_where_clusters_are_refused(tmp_path, limit):
     q_ref = s_ref - s_ref.sum() / t_ref.sum() * t_ref
     assert few["rel"].max() <= 1e-12
     assert np.abs(few["q"] - q_ref).max() <= 1e-8 * max(1.0, np.abs(q_ref).max())
+
+
+def test_static_solve_of_a_small_system_meets_in_one_block():
+    """Up to 112 atoms the solve is one block's. Twenty iterations on 24 rows took 0.76 times as long as on 129 rows on a cluster
+    while that block met as a cluster of one and divided twice. At most 0.7 times."""
+    import torch
+    import rxcuda
+    lib, err = rxcuda.load(), ctypes.create_string_buffer(256)
+    up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    took = []
+    for n in (24, 129):
+        rng = np.random.default_rng(n)   # a full matrix of condition 1e4: twenty iterations do not exhaust it
+        Q = np.linalg.qr(rng.normal(size=(n, n)))[0]
+        A = (Q * np.logspace(0.0, 4.0, n)) @ Q.T
+        rs = np.arange(0, n * (n - 1) + 1, n - 1, dtype=np.int32)
+        rows, col = np.nonzero(~np.eye(n, dtype=bool))
+        col, val, eta, chi = col.astype(np.int32), A[rows, col], np.diag(A).copy(), rng.uniform(-5.0, 5.0, size=n)
+        a = [up(x) for x in (rs, col, val, eta, chi)]
+        guess = torch.zeros((3, 20, n), dtype=torch.float64, device="cuda")   # s, t and q of every solve
+        it, rel = torch.zeros(2, dtype=torch.int32, device="cuda"), torch.zeros(2, dtype=torch.float64, device="cuda")
+        best = float("inf")
+        for _ in range(30):
+            guess.zero_()
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record()
+            for k in range(20):   # twenty iterations each
+                rc = lib.rx_qeq_solve_static(n, *(x.data_ptr() for x in a), *(guess[c, k].data_ptr() for c in range(3)), 1e-300, 21,
+                                             it.data_ptr(), rel.data_ptr(), torch.cuda.current_stream().cuda_stream, err, 256)
+                assert rc == 0, err.value.decode()
+            ev[1].record()
+            torch.cuda.synchronize()
+            best = min(best, ev[0].elapsed_time(ev[1]))
+        assert it.tolist() == [21, 21]
+        took.append(best)
+    assert took[0] <= 0.7 * took[1], took
 
 
 TIME_SOLVES = """
