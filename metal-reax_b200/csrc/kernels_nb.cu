@@ -596,17 +596,14 @@ __global__ void k_count_pairs(Dev d) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= d.na) return;
-  const SysInfo s = d.sys[d.sys_of[warp]];
-  const double4 xi = d.xr[warp];
-  const int i = ord_atom(xi), cnt = d.nbr_cnt[warp];
+  const int i = d.cell_atoms[warp], cnt = d.nbr_cnt[warp];
   const long long tag_i = d.tag[i];
   const int center = (d.S * d.S * d.S - 1) / 2;
   int counted = 0;
   for (int e = lane; e < cnt; e += 32) {
     const unsigned code = d.nbr[static_cast<size_t>(warp) * d.ncap + e];
     const int sidx = static_cast<int>(code >> d.abits);
-    const double4 xj = d.xr[code & d.amask];
-    const int j = ord_atom(xj);
+    const int pj = static_cast<int>(code & d.amask), j = d.cell_atoms[pj];
     if (sidx == center) {
       counted += j > i;
       continue;
@@ -617,7 +614,7 @@ __global__ void k_count_pairs(Dev d) {
       continue;
     }
     double dv[3];   // an image of i itself: the positive direction
-    pair_dvec_x(d, s, i, j, sidx, xi, xj, dv);
+    pair_dvec_x(d, d.sys[d.sys_of[warp]], i, j, sidx, d.xr[warp], d.xr[pj], dv);
     const double SMALL = 1e-4;
     counted += dv[2] > SMALL || (fabs(dv[2]) < SMALL && (dv[1] > SMALL || (fabs(dv[1]) < SMALL && dv[0] > SMALL)));
   }
