@@ -916,7 +916,9 @@ struct Context {
     if (nsys == 1 && na > tune.lone_grid_min) {   // one large system: all SMs on its rows, block partials in block order
       const int units = tune.cg_per_sm > 0 ? std::min(tune.cg_per_sm, 4) : 4;
       const int threads = 256 * units;
-      int grid = std::max(1, std::min(nsm, (na + (threads / 32) - 1) / (threads / 32)));
+      // a block per SM from two rows a block on: 41 blocks of 16 rows (648 atoms of water) met 2 us an iteration later than
+      // 148 blocks of 4 or 5, and below some 300 rows (100 atoms: 7 blocks 281 us, 100 blocks 373) a few blocks are quicker
+      const int grid = na >= 2 * nsm ? nsm : std::max(1, (na + (threads / 32) - 1) / (threads / 32));
       // the rows' vectors and lengths in shared memory where they fit beside the rings (108 bytes a row)
       const int rows = (na + grid - 1) / grid;
       const size_t rings = static_cast<size_t>(threads / 32) * kRingBytes, with_rows = rings + 108 * static_cast<size_t>(rows);

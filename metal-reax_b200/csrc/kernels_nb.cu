@@ -2,6 +2,7 @@
 #include <cooperative_groups.h>
 
 #include <type_traits>
+#include <utility>
 
 #include "device.cuh"
 #include "kernels.hpp"
@@ -986,6 +987,9 @@ __global__ void __launch_bounds__(1024, 1) k_cg_grid(Dev d, CgArgs a) {
       const bool in_s = act_s && it_s < a.imax && sqrt(sig_s) > stop_s;
       const bool in_t = act_t && it_t < a.imax && sqrt(sig_t) > stop_t;
       if (!in_s && !in_t) break;
+      // d.Ad = u.w - beta r.u / (the previous step length); beta is 0 on the first iteration from a residual
+      const double bs = in_s ? beta_s : 0.0, bt = in_t ? beta_t : 0.0;
+      const double less_s = fresh || !in_s ? 0.0 : bs * sig_s / alpha_s, less_t = fresh || !in_t ? 0.0 : bt * sig_t / alpha_t;
       // w = A u ; partial u.w
       fast.run(d.amask, r0 + w0, a.df, W + w0);
       __syncthreads();
@@ -1002,10 +1006,8 @@ __global__ void __launch_bounds__(1024, 1) k_cg_grid(Dev d, CgArgs a) {
       g.sync();
       grid_totals<2>(partbuf(), nb, tot, tot_sh);
       ++phase;
-      // d.Ad = u.w - beta r.u / (the previous step length); beta is 0 on the first iteration from a residual
-      const double bs = in_s ? beta_s : 0.0, bt = in_t ? beta_t : 0.0;
-      alpha_s = in_s ? sig_s / (fresh ? tot[0] : tot[0] - bs * sig_s / alpha_s) : 0.0;
-      alpha_t = in_t ? sig_t / (fresh ? tot[1] : tot[1] - bt * sig_t / alpha_t) : 0.0;
+      alpha_s = in_s ? sig_s / (tot[0] - less_s) : 0.0;
+      alpha_t = in_t ? sig_t / (tot[1] - less_t) : 0.0;
       if (!(isfinite(alpha_s) && isfinite(alpha_t))) { breakdown = true; break; }
       // d = u + beta d ; Ad = w + beta Ad ; x += alpha d ; r -= alpha Ad ; u = M^-1 r ; partial r.u
       loc[0] = loc[1] = 0.0;
@@ -1030,8 +1032,9 @@ __global__ void __launch_bounds__(1024, 1) k_cg_grid(Dev d, CgArgs a) {
         loc[0] += r.x * u.x; loc[1] += r.y * u.y;
       }
       block_partials<2>(loc, partbuf(), sh);
+      auto token = g.barrier_arrive();
       fast.start(d, r0 + w0, w1 - w0, cnt + w0, ring);
-      g.sync();
+      g.barrier_wait(std::move(token));
       grid_totals<2>(partbuf(), nb, tot, tot_sh);
       ++phase;
       if (in_s) { beta_s = tot[0] / sig_s; sig_s = tot[0]; ++it_s; }

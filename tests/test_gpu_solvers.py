@@ -303,6 +303,21 @@ def test_charge_solve_takes_the_quicker_kernel(tmp_path):
         assert rule[k] <= 1.2 * without[k], (k, float(rule[k]), float(without[k]))
 
 
+@pytest.mark.parametrize("n", [2, 33, 295, 296, 297, 600, 1999])
+def test_single_system_solve_of_small_systems(engine, oracle, n):
+    """The solve on all SMs below its usual sizes: blocks of one or two rows, some without rows, and both sides of 296 atoms
+    (two rows a block). As for the other sizes: 1e-10 e at tol 1e-12."""
+    s = _jittered(n, 300 + n)
+    engine.set_tuning("lone_grid_min", 0)
+    engine.set_systems([s])
+    engine.qeq_reset()
+    got = engine.qeq_solve()
+    engine.set_tuning("lone_grid_min", 4096)
+    ref = oracle.qeq(s, tol=1e-12, imax=400)
+    assert np.abs(got["q"] - ref["q"]).max() <= 1e-10
+    assert got["rel"].max() <= 1e-12
+
+
 def test_charge_solve_with_vectors_in_global_memory(engine):
     """A system of more rows per block than shared memory holds (its vectors stay in global memory), against the segmented
     FP64 solve of the same system. Both stop at a relative residual of 1e-10; diag(eta) + H has a condition number of a few
