@@ -233,10 +233,12 @@ int rx_update_systems(rx_context* ctx, int nkeep, const int* keep, int nnew, con
 int rx_md_targets(rx_context* ctx, const double* t_target, const int* active);
 
 /* Launch-shape tuning (no counterpart in the reference, whose Metal kernels use a fixed threadgroup of 64). All but
- * RX_TUNE_CG_BLOCKS_PER_SM leave every result bit unchanged. RX_TUNE_*_TPB: threads per block of a warp-per-atom kernel (64, 128, 256: atoms per
- * block x 32) or of the bonded kernels (32, 64, 128); RX_TUNE_LONE_GRID_MIN: a context holding one
- * system of more atoms takes the single-system CG (all SMs on its rows, default 4096; a batch always takes the
- * segmented CG, so a system alone and in a batch give the same bits only below this size); RX_TUNE_OVERLAP: 1 (the
+ * RX_TUNE_CG_BLOCKS_PER_SM and RX_TUNE_LONE_GRID_MIN leave every result bit unchanged. RX_TUNE_*_TPB: threads per block
+ * of a warp-per-atom kernel (64, 128, 256: atoms per block x 32) or of the bonded kernels (32, 64, 128);
+ * RX_TUNE_LONE_GRID_MIN: a context holding one system of more atoms takes the single-system CG (all SMs on its rows,
+ * default 4096). Every other system takes, whichever is expected to be quicker, a thread-block cluster (up to 4096 atoms)
+ * or the segmented CG (all SMs on the rows of every system); these two give the same bits, so a system alone and in a
+ * batch give the same bits up to this size; RX_TUNE_OVERLAP: 1 (the
  * default) runs the bonded terms, which need no charge, concurrently with the charge solve, 0 after it;
  * RX_TUNE_CG_BLOCKS_PER_SM: threads per SM of the single-system CG in units of 256, as one block per SM (1-4, default
  * 2, leaving room for the concurrent bonded terms; 0: four) - unlike the other keys this changes the order of the CG's sums, so the charges' last

@@ -807,8 +807,8 @@ struct Context {
     return a;
   }
 
-  // Launch shapes (atoms per block of the warp-per-atom and thread-per-atom kernels, the size above which a lone
-  // system takes the single-system CG): none changes a result bit, so rx_autotune may pick them by measurement.
+  // Launch shapes: threads per block of the warp-per-atom and bonded kernels (no result bit depends on them, so rx_autotune
+  // picks them by measurement), and the size above which a lone system takes the single-system CG.
   struct Tune {
     int tpb_pairs = 128, tpb_nb = 128, tpb_hb = 128, tpb_bonds = 128, tpb_atom = 64;
     int lone_grid_min = 4096;
@@ -821,7 +821,7 @@ struct Context {
     int cg_per_sm = 2;
   } tune;
   int grid_occ[5] = {0, 0, 0, 0, 0}, seg_per_sm = 0;
-  static constexpr int kCgSmem = 220 * 1024;   // dynamic shared memory of the single-system CG at most
+  static constexpr int kCgSmem = 220 * 1024;   // dynamic shared memory of the single-system and cluster CG at most
 
   // ---- the cluster solve's launch shape (no result bit depends on it)
   static constexpr int kClusterThreads = 512;
@@ -850,7 +850,10 @@ struct Context {
   // The cluster size with the shortest expected solve. An iteration of a system of n rows on c blocks takes about
   // kRowUs n / c + kMeetUs; the clusters share the systems, and none ends before the largest system's. Measured, us a
   // solve on 2, 4, 8, 16 blocks: 512 CHO systems of 64-1024 atoms 6925, 7235, 10885, 17918; 16 of 100-5000 (those up to
-  // 4096) 8: 2893, 16: 1542; one of 648 atoms 422, 250, 164, 116. 0 where the GPU holds no cluster of any size.
+  // 4096) 8: 2893, 16: 1542; one of 648 atoms 422, 250, 164, 116. Around the crossings, taken and next smaller, us a cold
+  // solve: 16 CHO systems of 100-2500 atoms 16: 1239, 8: 1720; 4 of 500 16: 641, 8: 885; 32 of 300-700 8: 1698, 4 or
+  // segmented 2700; 8 of water of 648 16: 932, 8: 732 (short rows: the estimate is of long ones). 0 where the GPU holds no
+  // cluster of any size.
   int cluster_size() {
     constexpr double kRowUs = 0.25, kMeetUs = 4.0;
     int best = 0;
@@ -929,7 +932,6 @@ struct Context {
         RXCU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&grid_occ[units], k_cg_grid, threads, kCgSmem));
       }
       if (grid_occ[units] < 1) throw Error(RX_ERR_CUDA, "the single-system CG block does not fit on an SM");
-      a.begin = 0;
       a.n = na;
       void* args[] = {const_cast<Dev*>(&d), &a};
       ++launches;
@@ -976,16 +978,17 @@ struct Context {
     toc(1);
   }
 
-  // After the Verlet check and rebuild, the bonded chain (bond orders, then k_bonded_atom, with the H-bonds on `side_h`
-  // and the torsions on `side_t`, then the bonded gathers k_fold and k_dbond) needs neither the neighbor rows nor the
-  // charges, so with tune.overlap it runs on `side` next to the row filter and the charge solve; the non-bonded pairs follow the charges on `stream`, and k_force_final joins both. Each branch writes its own arrays (fnb, vir_nb; bacc/bfn/fown; *_h; *_t, Tl), and
-  // all join before the gathers, which add them in fixed order, so the schedule changes no result bit. With timing
-  // on, every branch runs on `stream`, one after the other, so each phase is timed alone.
   // at most one listed slot per bond (the tag-order end): half the slots bound the list; the warps go through it in
   // strides, so that the many slots that are no central bond cost no blocks
   unsigned torsion_blocks(int tpb) const {
     return std::min(blocks((static_cast<long long>(na) * bcap + 1) / 2 * kLanes, tpb), static_cast<unsigned>(nsm * 2048 / tpb));
   }
+
+  // After the Verlet check and rebuild, the bonded chain (bond orders, then k_bonded_atom, with the H-bonds on `side_h`
+  // and the torsions on `side_t`, then the bonded gathers k_fold and k_dbond) needs neither the neighbor rows nor the
+  // charges, so with tune.overlap it runs on `side` next to the row filter and the charge solve; the non-bonded pairs follow the charges on `stream`, and k_force_final joins both. Each branch writes its own arrays (fnb, vir_nb; bacc/bfn/fown; *_h; *_t, Tl), and
+  // all join before the gathers, which add them in fixed order, so the schedule changes no result bit. With timing
+  // on, every branch runs on `stream`, one after the other, so each phase is timed alone.
   void launch_bonded(const Dev& d) {
     const bool conc = !timing;
     cudaStream_t bs = conc ? side : stream, hs = conc ? side_h : stream, ts = conc ? side_t : stream;

@@ -17,18 +17,18 @@ struct QeqParams {
   double tap[8];   // taper coefficients on [swa, swb]
 };
 
-// per-system state of the segmented (batched) CG
+// per-system state of the segmented CG
 struct SysCg {
   double sig_s, sig_t, bnorm_s, bnorm_t, alpha_s, alpha_t, beta_s, beta_t;
   int act_s, act_t, it_s, it_t, live, breakdown;
   unsigned counter;   // rows of this system that have arrived in the current pass
 };
 
-constexpr int kClusterAtoms = 4096;   // systems of up to this many atoms are solved by a thread-block cluster each
-constexpr int kRingBytes = 6144;   // shared memory per warp of the charge solve's row products (rows_stream)
+constexpr int kClusterAtoms = 4096;   // systems of up to this many atoms can be solved by a thread-block cluster each
+constexpr int kRingBytes = 6144;   // shared memory per warp of the charge solve's row products (RowStream)
 
 struct CgArgs {
-  int begin, n, imax;
+  int n, imax;
   double tol;
   double2* x;      // (s, t)
   double2* b;
@@ -38,7 +38,7 @@ struct CgArgs {
   double2* q;
   double2* s;      // A d (single-system CG)
   float2* df;      // FP32 copy of M^-1 r, gathered by the single-precision-matrix iterations (single-system CG)
-  int smem_rows;   // rows per block whose vectors its shared memory holds (single-system CG; 0: vectors in global memory)
+  int smem_rows;   // rows per block whose vectors its shared memory holds (single-system CG: 0 leaves them in global memory)
   double* eta;
   double* part;    // 2 * 8 * gridDim.x partial sums (double-buffered)
   int* out_iters;

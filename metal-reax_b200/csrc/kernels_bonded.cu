@@ -292,8 +292,8 @@ __global__ void k_atom_quantities(Dev d, DevFF ff) {
 // angles' order; per-atom sums are fixed exchanges. So every sum has one order. Against one thread per atom, k_bonded_atom
 // and k_hbond (each alone): 648 atoms of water 151 -> 44 us, 24,000 351 -> 180, 512 CHO systems 3.0 -> 1.6 ms, one CHO
 // system of 333 atoms 320 -> 50 us. At 168 registers three blocks of 128 threads fit an SM; 255 (no spills) or 128
-// measured the same within 5 %. (Handed over through shared memory
-// instead, the kernel's blocks found no room beside the charge solve's rings: plugin step of 24,000 atoms 1.21 -> 1.28 ms.)
+// measured the same within 5 %. (Handed over through shared memory instead, the kernel's blocks found no room beside the
+// charge solve's rings: plugin step of 24,000 atoms 1.21 -> 1.28 ms.)
 
 __device__ inline double lanes_sum(double v) {
 #pragma unroll

@@ -144,9 +144,9 @@ __device__ inline void taper_horner(const double* c, double r, double& Tap, doub
   dTap = g;
 }
 
-// Verlet rows (in cell order, entries by cell-order position), one warp per atom of a system being rebuilt: every image within nonb_cut + skin (a superset of the
-// owned-row cut-off of build_far_list, src/neighbor/neighbor.cpp:180-212). The cells within `range` of the atom's cell
-// are visited as runs of consecutive cells along x (one contiguous range of the cell-ordered atoms per run and periodic
+// Verlet rows (in cell order, entries by cell-order position), one warp per atom of a system being rebuilt: every image
+// within nonb_cut + skin (a superset of the owned-row cut-off of build_far_list, src/neighbor/neighbor.cpp:180-212). The
+// cells within `range` of the atom's cell are visited as runs of consecutive cells along x (one contiguous range of the cell-ordered atoms per run and periodic
 // image), so the candidate loads are coalesced. Entries are written through a warp ballot in visiting order
 // (deterministic). Rows only need to be supersets (every consumer re-tests its entries exactly in FP64 on the current
 // positions), so candidates are tested in single precision against the system's thresholds SysInfo::vthr, which add
@@ -908,8 +908,12 @@ __device__ inline void grid_totals(const double* part, int nblocks, double* tot,
 // only the copy `df` of u = M^-1 r. The iteration is the form of Chronopoulos and Gear (J. Comput. Appl. Math. 25, 153
 // (1989)): w = A u, then d = u + beta d and A d = w + beta (A d) by recurrence, so that only two grid barriers are
 // needed per iteration (after the row products, carrying u.w, and after the vector update, carrying the new r.u)
-// instead of three. Reductions are fixed-order, so the result is bitwise reproducible. Only grid.sync() waits; the
-// kernel is launched cooperatively.
+// instead of three. Reductions are fixed-order, so the result is bitwise reproducible. Only the grid barrier waits; the
+// kernel is launched cooperatively, with 256 to 1024 threads a block (hence the bound).
+//
+// Profiled (24,000 atoms of water, 512 threads): 30.8 us a matrix pass alone and cold, 27.9 MB from DRAM; stalls an issue:
+// fixed latencies 2.8, barriers 2.4, shared memory and conversions 1.3, gathers 0.6; the conversions of the matrix take
+// 28 % of their pipe, FP64 7 %. So it waits for instruction latencies and barriers with 16 warps an SM, not for memory.
 constexpr double kRefineDrop = 1e-6;
 
 __global__ void __launch_bounds__(1024, 1) k_cg_grid(Dev d, CgArgs a) {
@@ -1089,6 +1093,11 @@ __global__ void __launch_bounds__(1024, 1) k_cg_grid(Dev d, CgArgs a) {
 // A system's bits do not depend on the size of the cluster or on what else is in the batch: a row product depends on
 // the row alone, and every dot product is summed over groups of eight consecutive rows (a fixed exchange), the groups'
 // sums being handed to every block of the cluster and added up in one fixed order.
+//
+// Profiled (648 atoms on 16 blocks, 64 CHO systems on 120 blocks): 16 warps an SM, stalls an issue: fixed latencies 2.5,
+// barriers 1.8-2.0, shared memory and conversions 1.6, gathers 0.6; FP64 pipe 8 %, conversions 12 %: too few warps to
+// cover the latencies. A second block does not fit an SM (96 KB of rings and 24 KB of sums each); the bound of two keeps
+// the registers at 64 a thread, so that half of them are left to the bonded terms that run beside the solve.
 constexpr int kGroup = 8;   // rows whose terms are summed before they are handed over
 __global__ void __launch_bounds__(512, 2) k_cg_cluster(Dev d, CgArgs a) {
   cg::cluster_group cl = cg::this_cluster();

@@ -44,7 +44,8 @@ void put_err(char* err, int errlen, const char* msg) {
 }
 
 // One row of (diag(eta) + H) v for both right-hand sides, a warp per row. kFlight entries per lane are loaded before the
-// first gather is waited for: a row product is bound by the latency of its dependent index -> vector loads.
+// first gather is waited for: a row product is bound by the latency of its dependent index -> vector loads. 3, 4, 5, 6 and 8
+// in flight, us a solve: 2592 atoms of water 1083, 1059, 1093, 1080, 1175; 12,000 3576, 3543, 3336, 3744, 3444.
 constexpr int kFlight = 5;
 __device__ inline double2 csr_row_mv(int i, const int* __restrict__ rs, const int* __restrict__ col, const double* __restrict__ val,
                                      double eta, const double2* v) {

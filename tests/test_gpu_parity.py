@@ -533,8 +533,7 @@ def test_half_pair_nonbonded_matches_full_rows(engine):
     """The step's non-bonded kernel computes each pair once and hands the partner its share through the fixed-point
     accumulator; the full-row kernel (taken for per-atom tallies) computes every pair from both ends. Same pairs and the
     same FP32 terms, so energies agree to summation order and the census is identical; the gradients agree to FP32
-    rounding (1e-6 of the largest component), because the two ends of a pair round the charge product and the type-pair
-    constants in their own order, so the full-row kernel's two shares of a pair differ in their last bits."""
+    rounding (1e-6 of the largest component)."""
     for s in small_systems()[:3] + [__import__("systems").water_box(8)]:
         q = fixed_charges(s)
         engine.set_systems([s])
