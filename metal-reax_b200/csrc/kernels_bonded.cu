@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(128, 3) k_bonded_atom(Dev d, DevFF ff, DevCtl 
           }
         }
       }
-      // the lane that owns a bond adds what this round's angles give it, in the angles' order. Rounds without an angle end
+      // the lane that owns a bond adds what these angles give it, in the angles' order. Passes without an angle end
       // here; the vote also brings the lanes together again before the exchange: without it the kernel took 1158 us
       // instead of 113 on 1000 CHO atoms of which one has 17 bonds (two passes of the loop below: 105 and 100 us on 15)
       if (!__any_sync(0xffffffffu, o.pi >= 0)) continue;
@@ -1033,7 +1033,7 @@ __global__ void __launch_bounds__(128, 3) k_torsion(Dev d, DevFF ff, DevCtl ctl)
           vir_add(vir, pl, gl);
         }
       }();
-      // the lane that owns a row adds what this round's combinations give it, in their order
+      // the lane that owns a row adds what these combinations give it, in their order
       if (!__any_sync(0xffffffffu, o.pi >= 0)) continue;
       for (int k0 = 0; k0 < most; ++k0) {
         const int k = k0 * kLanes + g;
